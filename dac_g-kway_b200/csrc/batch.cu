@@ -501,6 +501,23 @@ bool partition_batch_union(Handle& hh, const DevGraph& hg, i32 G, const i32* gra
     gb.gk = gk_d;
     gb.part_base = pbase_d;
     gb.depth = depth;
+    // the bisections of every depth, all graphs together
+    std::vector<int2> level, subs;
+    for (i32 i = 0; i < G; ++i) level.push_back(make_int2(pb[i], pb[i] + kv[i]));
+    for (i32 d = 0; d < depth; ++d) {
+      gb.sub_ptr.push_back((i32)subs.size());
+      std::vector<int2> next;
+      for (const int2 q : level) {
+        if (q.y - q.x < 2) continue;
+        subs.push_back(q);
+        const i32 pm = q.x + (q.y - q.x) / 2;
+        next.push_back(make_int2(q.x, pm));
+        next.push_back(make_int2(pm, q.y));
+      }
+      level.swap(next);
+    }
+    gb.sub_ptr.push_back((i32)subs.size());
+    gb.subs = to_dev(hh, subs);
     device_init_partition(hh, cu.g, K, o.eps, o.seed, std::max(1, std::min(8, o.init_trials)), part_cu, &gb);
   }
   refine_init_union(hh, rc, cu.g, part_cu, bnd_cu);   // boundary of the initial parts, part weights

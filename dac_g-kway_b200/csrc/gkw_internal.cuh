@@ -378,6 +378,8 @@ struct GggpBatch {
   const i32* part_v0 = nullptr;     // [parts] vertex range of the part's graph
   const i32* part_v1 = nullptr;
   i32 depth = 0;                    // recursion depth of the largest k
+  const int2* subs = nullptr;       // (p0, p1) of the sub-problems with two or more parts, by depth
+  std::vector<i32> sub_ptr;         // [depth + 1] first of each depth in subs
 };
 void device_init_partition(Handle& h, const DevGraph& g, i32 k, double eps, u64 seed, i32 trials,
                            i32* d_part, const GggpBatch* batch = nullptr);
