@@ -1106,6 +1106,372 @@ __device__ i32 select_sort(const LevelArgs& a, const u64* cands, i32 cnt, u64* s
   return B;
 }
 
+// ---------------------------------------------------------------------------
+// The first B candidates in order, and the largest balanced index, without a
+// comparison sort.  Both run on every CTA that owns a move index, so they are
+// a chain every round waits for: for the 27-point grid's ~4600 candidates a
+// round at k = 64 the threshold search, merge sorts and event sort below
+// (select_sort, refine_balanced_pos) took 56 us of a 90 us round.
+//
+// rank_select: a bucket sort.  Gains are counted in bins (one bin a gain below
+// 512, 16 bins an octave above); the bin where the count reaches B ends the
+// kept set.  Each kept bin then gets as many buckets as it has keys (at most
+// kRankSub), split by vertex id -- bins of several gains by gain -- and a key's
+// rank is its bucket's start plus the smaller keys in the bucket.  Returns
+// false (block-uniform) when the buckets come out too uneven; the caller then
+// sorts.  keep[r] is the key of rank r < B, kidx[r] its place in the list.
+// ---------------------------------------------------------------------------
+constexpr i32 kRankBins = 1024;      // gain bins
+constexpr i32 kRankBuckets = 3072;
+constexpr i32 kRankSub = 1024;       // buckets of one gain bin
+constexpr i32 kRankDeep = 192;       // most keys of one bucket
+constexpr i32 kRankSlots = kMaxMoveCap + 256;   // kept keys: B - 1 and one bucket at most
+static_assert(kRankDeep <= 256 && kRankSlots <= kSortMax, "the slots fit the sort buffer");
+static_assert(kMaxMoveCap + 2 * kRankBins + kRankBuckets + kRankSlots <= kGreedyWords,
+              "the rank tables fit the greedy region");
+static_assert(kMaxMoveCap + kRankSub <= kRankBuckets, "kept bins' buckets fit");
+static_assert(kRankBins % kLevelThreads == 0 && kRankBuckets % kLevelThreads == 0, "scans split evenly");
+
+__device__ __forceinline__ u32 rank_gain(u64 key) { return 0x7fffffffu - (u32)(key >> 32); }   // positive
+__device__ __forceinline__ i32 rank_bin(u32 g) {
+  if (g < 512u) return 863 - (i32)g;
+  const int e = 31 - __clz(g);
+  return 863 - (512 + (e - 9) * 16 + (i32)((g >> (e - 4)) & 15u));
+}
+// bucket of a key among its bin's nsub (monotone in the key's order): the id,
+// or in bins of several gains the gain, as a fraction of its range
+__device__ __forceinline__ i32 rank_sub(u32 g, u32 id, i32 nsub, int id_bits) {
+  if (g < 512u) return (i32)__umulhi(id << (32 - id_bits), (u32)nsub);
+  const int sh = 27 - __clz(g);
+  const u32 low = (1u << sh) - 1u;
+  return (i32)__umulhi((low - (g & low)) << (32 - sh), (u32)nsub);
+}
+
+__device__ __noinline__ bool rank_select(const u64* cands, i32 cnt, i32 B, i32 id_lo, i32 id_n) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ i32 s_total, s_deep;
+  __shared__ u32 s_warp[33];
+  u64* s = reinterpret_cast<u64*>(smem_raw);                              // [kRankSlots]
+  unsigned short* sb = reinterpret_cast<unsigned short*>(s + kRankSlots);   // [kRankSlots] bucket of slot
+  i32* greedy = reinterpret_cast<i32*>(smem_raw + kSortMax * 8);
+  u64* keep = reinterpret_cast<u64*>(greedy + kGreedyWords);
+  i32* kidx = greedy;                 // [kMaxMoveCap]
+  i32* bins = kidx + kMaxMoveCap;     // [kRankBins] counts, then first bucket
+  i32* nsub = bins + kRankBins;       // [kRankBins] buckets of the bin
+  i32* bucket = nsub + kRankBins;     // [kRankBuckets] counts, then fill positions
+  i32* sidx = bucket + kRankBuckets;  // [kRankSlots] list place of slot
+  static_assert(kRankSlots * 10 <= kSortMax * 8, "keys and buckets of the slots fit the sort buffer");
+  constexpr i32 kReg = 8;             // keys per thread kept in registers
+  const i32 T = (i32)blockDim.x;
+  int id_bits = 1;
+  while (((i64)1 << id_bits) < id_n) ++id_bits;
+  u64 rk[kReg];
+#pragma unroll
+  for (i32 q = 0; q < kReg; ++q) rk[q] = (i32)threadIdx.x + q * T < cnt ? ldc(cands + threadIdx.x + q * T) : 0ull;
+  auto each = [&](auto f) {   // f(list place, key) for this thread's keys
+#pragma unroll
+    for (i32 q = 0; q < kReg; ++q)
+      if ((i32)threadIdx.x + q * T < cnt) f((i32)threadIdx.x + q * T, rk[q]);
+    for (i32 i = (i32)threadIdx.x + kReg * T; i < cnt; i += T) f(i, ldc(cands + i));
+  };
+  for (i32 b = threadIdx.x; b < kRankBins; b += T) bins[b] = 0;
+  for (i32 b = threadIdx.x; b < kRankBuckets; b += T) bucket[b] = 0;
+  if (threadIdx.x == 0) s_deep = 0;
+  __syncthreads();
+  each([&](i32, u64 key) { atomicAdd(&bins[rank_bin(rank_gain(key))], 1); });
+  __syncthreads();
+  // kept bins: all whose first key has a rank below B
+  {
+    constexpr i32 kPer = kRankBins / kLevelThreads;
+    const i32 b0 = threadIdx.x * kPer;
+    i32 c[kPer];
+    u32 loc = 0;
+#pragma unroll
+    for (i32 j = 0; j < kPer; ++j) {
+      c[j] = bins[b0 + j];
+      loc += (u32)c[j];
+    }
+    u32 tot;
+    u32 run = block_exscan_u32(loc, s_warp, tot);
+    u32 subs = 0;
+#pragma unroll
+    for (i32 j = 0; j < kPer; ++j) {
+      const bool in = run < (u32)B && c[j] > 0;
+      c[j] = in ? c[j] : 0;
+      run += (u32)c[j];
+      subs += (u32)(c[j] < kRankSub ? c[j] : kRankSub);
+    }
+    u32 base = block_exscan_u32(subs, s_warp, tot);
+#pragma unroll
+    for (i32 j = 0; j < kPer; ++j) {
+      const i32 ns = c[j] < kRankSub ? c[j] : kRankSub;
+      bins[b0 + j] = (i32)base;
+      nsub[b0 + j] = ns;
+      base += (u32)ns;
+    }
+  }
+  __syncthreads();
+  auto bucket_of = [&](u64 key) -> i32 {   // -1: not in a kept bin
+    const u32 g = rank_gain(key);
+    const i32 b = rank_bin(g), ns = nsub[b];
+    return ns ? bins[b] + rank_sub(g, (u32)key - (u32)id_lo, ns, id_bits) : -1;
+  };
+  each([&](i32, u64 key) {
+    const i32 x = bucket_of(key);
+    if (x >= 0) atomicAdd(&bucket[x], 1);
+  });
+  __syncthreads();
+  // bucket starts; kept buckets start below rank B
+  {
+    constexpr i32 kPer = kRankBuckets / kLevelThreads;
+    const i32 b0 = threadIdx.x * kPer;
+    i32 c[kPer];
+    u32 loc = 0;
+#pragma unroll
+    for (i32 j = 0; j < kPer; ++j) {
+      c[j] = bucket[b0 + j];
+      loc += (u32)c[j];
+    }
+    u32 tot;
+    u32 run = block_exscan_u32(loc, s_warp, tot);
+    i32 deep = 0;
+#pragma unroll
+    for (i32 j = 0; j < kPer; ++j) {
+      const bool in = run < (u32)B;
+      bucket[b0 + j] = in ? (i32)run : -1;
+      if (in) deep = c[j] > deep ? c[j] : deep;
+      if (in && run + (u32)c[j] >= (u32)B) s_total = (i32)(run + (u32)c[j]);   // one bucket: the rest start at B or later
+      run += (u32)c[j];
+    }
+    deep = (i32)__reduce_max_sync(kFullMask, (u32)deep);
+    if ((threadIdx.x & 31) == 0 && deep > kRankDeep) s_deep = 1;
+  }
+  __syncthreads();
+  if (s_deep) return false;   // block-uniform; else s_total < B + kRankDeep
+  each([&](i32 i, u64 key) {
+    const i32 x = bucket_of(key);
+    if (x < 0 || bucket[x] < 0) return;
+    const i32 at = atomicAdd(&bucket[x], 1);
+    s[at] = key;
+    sb[at] = (unsigned short)x;
+    sidx[at] = i;
+  });
+  __syncthreads();
+  // rank within the bucket: its slots end at the fill position, and start
+  // where the bucket before it (any bucket: the fills are cumulative) ends
+  const i32 total = s_total;
+  for (i32 e = threadIdx.x; e < total; e += T) {
+    const u64 key = s[e];
+    const i32 x = sb[e];
+    const i32 hi = bucket[x], lo = x ? bucket[x - 1] : 0;
+    i32 r = lo;
+    for (i32 f = lo; f < hi; ++f) r += s[f] < key;
+    if (r < B) {
+      keep[r] = key;
+      kidx[r] = sidx[e];
+    }
+  }
+  __syncthreads();
+  return true;
+}
+
+// Largest balanced index of the ranked moves keep[0..B) (the rule of
+// refine_balanced_pos): moves into and out of parts that could pass MAXW are
+// events (part, rank, +-w), grouped by part with a counting sort; a part's
+// running change after one of its events is the sum of its events up to that
+// rank and holds until its next event; an event whose change is positive and
+// passes MAXW marks the ranks up to the next.  Parts in [pb, pb + k), k <=
+// kRankParts.  Neither function is inlined, so that the level kernel keeps its
+// registers; the arrays' addresses come in shared memory (a reference to the
+// kernel's arguments would move those to local memory: every phase 1.5x
+// slower) and the buffers are the kernel's dynamic shared memory.  Together
+// they take 23-25 us for the grid's candidates, 18 us for the 1100 of a
+// 4M-vertex circuit graph at k = 256 (45 us sorted).
+constexpr i32 kRankParts = 1024;
+struct RankedMoves {
+  // plain levels: list entries and the parts that could pass MAXW at all
+  const u64* cinfo;
+  const i32* cw;
+  const u32* risk;      // null: batched, every part may, and the moves' data by vertex
+  const i32 *part, *target, *vwgt;
+  const u32* pw;
+  const float* pmaxw;   // batched: MAXW of each part
+  float maxw;
+};
+
+__device__ __noinline__ i32 ranked_balanced_pos(const RankedMoves* mp, i32 B, i32 pb, i32 k) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ u32 s_warp[33];
+  i32* greedy = reinterpret_cast<i32*>(smem_raw + kSortMax * 8);
+  const u64* keep = reinterpret_cast<const u64*>(greedy + kGreedyWords);
+  const RankedMoves m = *mp;
+  constexpr i32 kLarge = 96;   // events of a part above which it is scanned instead
+  __shared__ i32 s_best, s_nlarge, s_large[2 * kMaxMoveCap / kLarge + 1];
+  const i32 T = (i32)blockDim.x;
+  i32* rflag = reinterpret_cast<i32*>(smem_raw);   // [kRankParts]
+  i32* rpw = rflag + kRankParts;            // [kRankParts] part weight before the round
+  i32* bcnt = rpw + kRankParts;             // [kRankParts] events of the part
+  i32* boff = bcnt + kRankParts;            // [kRankParts] first event, then one past the last
+  i32* diff = boff + kRankParts;            // [kMaxMoveCap]
+  i32* mw = diff + kMaxMoveCap;             // [kMaxMoveCap] weight of each move
+  static_assert(4 * kRankParts + 2 * kMaxMoveCap <= 2 * kSortMax, "part tables and moves fit the sort buffer");
+  u32* msd = reinterpret_cast<u32*>(greedy);   // [kMaxMoveCap] source << 16 | destination, in kidx's place
+  int2* ev = reinterpret_cast<int2*>(greedy + kMaxMoveCap);   // [2 * kMaxMoveCap] grouped events (rank, +-weight)
+  static_assert(5 * kMaxMoveCap <= kGreedyWords, "events fit the greedy region");
+  static_assert(kRankParts <= 65536 && kMaxMoveCap <= 65536, "16-bit parts and ranks");
+  for (i32 p = threadIdx.x; p < k; p += T) {
+    rflag[p] = m.risk ? ldc(m.risk + p) != 0 : 1;
+    rpw[p] = (i32)ldc(m.pw + pb + p);
+    bcnt[p] = 0;
+  }
+  for (i32 j = threadIdx.x; j < B; j += T) diff[j] = 0;
+  if (threadIdx.x == 0) {
+    s_best = 0;
+    s_nlarge = 0;
+  }
+  __syncthreads();
+  constexpr i32 kPer = kMaxMoveCap / kLevelThreads;   // moves per thread, their loads issued together
+  {
+    i32 at[kPer], ms[kPer], md[kPer], mv[kPer];
+#pragma unroll
+    for (i32 q = 0; q < kPer; ++q) {
+      const i32 j = (i32)threadIdx.x + q * T;
+      at[q] = j < B ? (m.risk ? greedy[j] : (i32)(u32)keep[j]) : 0;   // kidx, or the vertex
+    }
+#pragma unroll
+    for (i32 q = 0; q < kPer; ++q) {
+      ms[q] = md[q] = mv[q] = 0;
+      if ((i32)threadIdx.x + q * T < B) {
+        if (m.risk) {
+          const u64 inf = ldc(m.cinfo + at[q]);
+          mv[q] = ldc(m.cw + at[q]);
+          ms[q] = (i32)(u32)(inf >> 32);
+          md[q] = (i32)(u32)inf;
+        } else {
+          ms[q] = ldc(m.part + at[q]) - pb;
+          md[q] = ldc(m.target + at[q]) - pb;
+          mv[q] = m.vwgt[at[q]];
+        }
+      }
+    }
+#pragma unroll
+    for (i32 q = 0; q < kPer; ++q) {
+      const i32 j = (i32)threadIdx.x + q * T;
+      if (j < B) {
+        mw[j] = mv[q];
+        msd[j] = ((u32)ms[q] << 16) | (u32)md[q];
+        if (rflag[ms[q]]) atomicAdd(&bcnt[ms[q]], 1);
+        if (rflag[md[q]]) atomicAdd(&bcnt[md[q]], 1);
+      }
+    }
+  }
+  __syncthreads();
+  {   // first event of each part
+    const i32 b0 = 2 * (i32)threadIdx.x;
+    const u32 c0 = b0 < k ? (u32)bcnt[b0] : 0u, c1 = b0 + 1 < k ? (u32)bcnt[b0 + 1] : 0u;
+    u32 tot;
+    const u32 ex = block_exscan_u32(c0 + c1, s_warp, tot);
+    if (b0 < k) boff[b0] = (i32)ex;
+    if (b0 + 1 < k) boff[b0 + 1] = (i32)(ex + c0);
+    if (c0 > (u32)kLarge) s_large[atomicAdd(&s_nlarge, 1)] = b0;
+    if (c1 > (u32)kLarge) s_large[atomicAdd(&s_nlarge, 1)] = b0 + 1;
+  }
+  __syncthreads();
+  for (i32 j = threadIdx.x; j < B; j += T) {
+    const i32 sp = (i32)(msd[j] >> 16), dp = (i32)(msd[j] & 0xffffu), w = mw[j];
+    if (rflag[sp]) {
+      ev[atomicAdd(&boff[sp], 1)] = make_int2(j, -w);
+    }
+    if (rflag[dp]) {
+      ev[atomicAdd(&boff[dp], 1)] = make_int2(j, w);
+    }
+  }
+  __syncthreads();
+  for (i32 q = threadIdx.x; q < 2 * B; q += T) {   // the event of move q / 2 at its destination or source
+    const i32 j = q >> 1;
+    const i32 p = (i32)((q & 1) ? msd[j] >> 16 : msd[j] & 0xffffu);
+    if (!rflag[p] || bcnt[p] > kLarge) continue;
+    i32 D = 0, next = B;
+    const i32 fe = boff[p];
+#pragma unroll 4
+    for (i32 f = fe - bcnt[p]; f < fe; ++f) {
+      const int2 x = ev[f];
+      D += x.x <= j ? x.y : 0;
+      next = x.x > j && x.x < next ? x.x : next;
+    }
+    const float mxw = m.pmaxw ? __ldg(m.pmaxw + pb + p) : m.maxw;
+    if (D > 0 && __uint2float_rn((u32)D + (u32)rpw[p]) > mxw) {
+      atomicAdd(&diff[j], 1);
+      if (next < B) atomicAdd(&diff[next], -1);
+    }
+  }
+  // a part with many events: its running change at every rank by one scan
+  // (its events' pairwise sums are quadratic: 15-22 us of the check without)
+  {
+    const i32 lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    constexpr i32 kR = kPer;
+    const i32 R = (B + T - 1) / T;
+    const i32 j0 = (i32)threadIdx.x * R;
+    for (i32 x = 0; x < s_nlarge; ++x) {   // block-uniform
+      const i32 p = s_large[x];
+      const float mxw = m.pmaxw ? __ldg(m.pmaxw + pb + p) : m.maxw;
+      const u32 pw0 = (u32)rpw[p];
+      i32 val[kR];
+      i32 acc = 0;
+#pragma unroll
+      for (i32 r = 0; r < kR; ++r) {
+        const i32 j = j0 + r;
+        if (r < R && j < B) {
+          const u32 sd = msd[j];
+          const i32 w = mw[j];
+          acc += (i32)(sd & 0xffffu) == p ? w : (i32)(sd >> 16) == p ? -w : 0;
+        }
+        val[r] = acc;
+      }
+      i32 inc = acc;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const i32 y = __shfl_up_sync(kFullMask, inc, o);
+        if (lane >= o) inc += y;
+      }
+      u32* wsum = s_warp + (x & 1) * 16;   // alternating rows: one barrier per part
+      if (lane == 31) wsum[wid] = (u32)inc;
+      __syncthreads();
+      i32 before = inc - acc;
+      for (i32 w = 0; w < wid; ++w) before += (i32)wsum[w];
+#pragma unroll
+      for (i32 r = 0; r < kR; ++r) {
+        const i32 j = j0 + r;
+        const i32 D = before + val[r];
+        if (r < R && j < B && D > 0 && __uint2float_rn((u32)D + pw0) > mxw) {
+          atomicAdd(&diff[j], 1);
+          if (j + 1 < B) atomicAdd(&diff[j + 1], -1);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  // marks per rank = prefix of diff; the largest rank with none (0 if all are
+  // marked: move 0 is applied regardless)
+  const i32 R2 = (B + T - 1) / T;
+  const i32 j0 = (i32)threadIdx.x * R2;
+  u32 loc = 0;
+  for (i32 j = j0; j < j0 + R2 && j < B; ++j) loc += (u32)diff[j];
+  u32 tot;
+  i32 run = (i32)block_exscan_u32(loc, s_warp, tot);
+  i32 best = 0;
+  for (i32 j = j0; j < j0 + R2 && j < B; ++j) {
+    run += diff[j];
+    if (run == 0) best = j;
+  }
+  best = (i32)__reduce_max_sync(kFullMask, (u32)best);
+  if ((threadIdx.x & 31) == 0 && best) atomicMax(&s_best, best);
+  __syncthreads();
+  const i32 pos = s_best;
+  __syncthreads();
+  return pos;
+}
+
 // Balance rounds: greedy pass in sorted order over s[0..B): take a move while
 // its source is still overweight and its destination stays within the cap,
 // skip the others.  Sources and destinations of one round are disjoint (a
@@ -1170,7 +1536,8 @@ __device__ void ph_bal_select(const LevelArgs& a, u64* s, i32* greedy) {
 // candidate buckets and appends the moves it keeps to the flat list
 // top[0..mcount).  A graph with candidates raises anyf[r % 3]; block 0
 // clears anyf[(r + 1) % 3], last read two barriers ago.
-__device__ void ph_select_batch(const LevelArgs& a, u64* s, i32* greedy, u32* s_warp, bool balance_mode, i64 r) {
+__device__ void ph_select_batch(const LevelArgs& a, u64* s, i32* greedy, u64* s_keep, u32* s_warp,
+                                const RankedMoves* ranked, bool balance_mode, i64 r) {
   __shared__ i32 s_cnt, s_base;
   RoundState* st = a.st;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1187,15 +1554,23 @@ __device__ void ph_select_batch(const LevelArgs& a, u64* s, i32* greedy, u32* s_
     __syncthreads();
     if (cnt == 0) continue;   // block-uniform
     if (threadIdx.x == 0) atomicExch(a.anyf + r % 3, 1);
-    u64* cg = a.cands + __ldg(a.gvbase + g);
-    const i32 B = select_sort(a, cg, cnt, s, greedy);
+    const i32 v0 = __ldg(a.gvbase + g);
+    u64* cg = a.cands + v0;
+    const i32 pb = __ldg(a.gpbase + g), kg = __ldg(a.gk + g);
+    i32 B = cnt < a.move_cap ? cnt : a.move_cap;
     i32 keep;
-    if (!balance_mode) {
+    if (!balance_mode && kg <= kRankParts &&
+        rank_select(cg, cnt, B, v0, __ldg(a.gvbase + g + 1) - v0)) {
+      keep = ranked_balanced_pos(ranked, B, pb, kg) + 1;
+      for (i32 i = threadIdx.x; i < keep; i += blockDim.x) cg[i] = s_keep[i];
+    } else if (!balance_mode) {
+      B = select_sort(a, cg, cnt, s, greedy);
       // the check below overwrites s: park the sorted moves in the bucket
       for (i32 i = threadIdx.x; i < B; i += blockDim.x) cg[i] = s[i];
       keep = refine_balanced_pos(a, s, reinterpret_cast<u64*>(greedy), B, s_warp, a.part) + 1;
     } else {
-      keep = select_greedy(a, s, greedy, B, __ldg(a.gpbase + g), __ldg(a.gk + g));
+      B = select_sort(a, cg, cnt, s, greedy);
+      keep = select_greedy(a, s, greedy, B, pb, kg);
       for (i32 i = threadIdx.x; i < keep; i += blockDim.x) cg[i] = s[i];
     }
     if (threadIdx.x == 0) s_base = atomicAdd(a.mcount, keep);
@@ -1483,7 +1858,7 @@ __device__ bool refine_check_risk(const LevelArgs& a, i32 cnt, u64* s, i32* gree
 // count), so a CTA owns an index below B iff blockIdx.x * warps_per_cta < B.
 // Returns (thread 0) the CTA's appends to U.  cnt: the round's candidates.
 __device__ u32 ph_refine_apply(const LevelArgs& a, u64* s, i32* greedy, u64* keep, u32* s_warp, u64* s_tmp,
-                               UStage& S, i32 cnt) {
+                               const RankedMoves* ranked, UStage& S, i32 cnt) {
   RoundState* st = a.st;
   const i32 B = cnt < a.move_cap ? cnt : a.move_cap;
   const i32 nw = blockDim.x >> 5;
@@ -1507,6 +1882,14 @@ __device__ u32 ph_refine_apply(const LevelArgs& a, u64* s, i32* greedy, u64* kee
     bool done = false;
     if (cnt <= a.move_cap) done = refine_check_risk(a, cnt, s, greedy, keep, s_tmp, s_warp, &kstar, &napplied);
     trace_mark(a, 25);
+    if (!done && a.k <= kRankParts && rank_select(a.cands, cnt, B, 0, a.n)) {
+      trace_mark(a, 28);
+      pos = ranked_balanced_pos(ranked, B, 0, a.k);
+      napplied = pos + 1;
+      sorted = true;
+      done = true;
+      trace_mark(a, 27);
+    }
     if (!done) {
       select_sort(a, a.cands, cnt, s, greedy);   // s[0..B) sorted (ends with a block barrier)
       for (i32 i = threadIdx.x; i < B; i += blockDim.x) keep[i] = s[i];
@@ -1517,8 +1900,11 @@ __device__ u32 ph_refine_apply(const LevelArgs& a, u64* s, i32* greedy, u64* kee
       trace_mark(a, 26);
     }
   } else if (cnt > a.move_cap) {
-    select_sort(a, a.cands, cnt, s, greedy);   // the first cap candidates, all balanced
-    for (i32 i = threadIdx.x; i < B; i += blockDim.x) keep[i] = s[i];
+    // the first cap candidates, all balanced
+    if (!rank_select(a.cands, cnt, B, 0, a.n)) {
+      select_sort(a, a.cands, cnt, s, greedy);
+      for (i32 i = threadIdx.x; i < B; i += blockDim.x) keep[i] = s[i];
+    }
     sorted = true;
   }
   __syncthreads();
@@ -1800,6 +2186,10 @@ __global__ void __launch_bounds__(kLevelThreads, GKW_LEVEL_MIN_BLOCKS) k_level(L
   __shared__ i32 s_flag;
   __shared__ i32 s_cnt, s_base;
   __shared__ UStage s_ustage;
+  __shared__ RankedMoves s_ranked;
+  if (threadIdx.x == 0)
+    s_ranked = a.batch ? RankedMoves{nullptr, nullptr, nullptr, a.part, a.target, a.vwgt, a.pw, a.pmaxw, 0.f}
+                       : RankedMoves{a.cinfo, a.cw, a.risk, nullptr, nullptr, nullptr, a.pw, nullptr, a.maxw};
   {
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (wid < a.acc_warps)
@@ -1854,7 +2244,7 @@ __global__ void __launch_bounds__(kLevelThreads, GKW_LEVEL_MIN_BLOCKS) k_level(L
       ph_bal_emit(a);
       if (!grid_barrier(a.bar, a.err, &s_flag)) return;
       trace_mark(a, 11);
-      if (a.batch) ph_select_batch(a, s_sort, greedy, s_warp, true, fr);
+      if (a.batch) ph_select_batch(a, s_sort, greedy, s_keep, s_warp, &s_ranked, true, fr);
       else ph_bal_select(a, s_sort, greedy);
       if (!grid_barrier(a.bar, a.err, &s_flag)) return;
       trace_mark(a, 12);
@@ -1890,7 +2280,7 @@ __global__ void __launch_bounds__(kLevelThreads, GKW_LEVEL_MIN_BLOCKS) k_level(L
         if (!grid_barrier(a.bar, a.err, &s_flag)) return;
         trace_mark(a, 20);
         ++fr;
-        ph_select_batch(a, s_sort, greedy, s_warp, false, fr);
+        ph_select_batch(a, s_sort, greedy, s_keep, s_warp, &s_ranked, false, fr);
         if (!grid_barrier(a.bar, a.err, &s_flag)) return;
         trace_mark(a, 21);
         if (ldc(a.anyf + fr % 3) == 0) break;
@@ -1907,7 +2297,7 @@ __global__ void __launch_bounds__(kLevelThreads, GKW_LEVEL_MIN_BLOCKS) k_level(L
       if (nC < 0) nC = ldc(&st->ccount);
       trace_mark(a, 20);
       if (nC == 0) break;   // every CTA has the same count
-      const u32 my_u = ph_refine_apply(a, s_sort, greedy, s_keep, s_warp, s_tmp, s_ustage, nC);
+      const u32 my_u = ph_refine_apply(a, s_sort, greedy, s_keep, s_warp, s_tmp, &s_ranked, s_ustage, nC);
       if (!grid_barrier_count(a.cbar, cbk++, a.err, &s_flag, &s_total, my_u, &nU)) return;
       trace_mark(a, 23);
       const u32 my_p = ph_update(a, acc_all, true, s_ustage, nU);
