@@ -2171,11 +2171,12 @@ __device__ void ph_apply_balance(const LevelArgs& a, UStage& S) {
 // ---------------------------------------------------------------------------
 // The level kernel.
 // ---------------------------------------------------------------------------
-// Resident level-kernel CTAs per SM the register budget is sized for.
-#ifndef GKW_LEVEL_MIN_BLOCKS
-#define GKW_LEVEL_MIN_BLOCKS 2
-#endif
-__global__ void __launch_bounds__(kLevelThreads, GKW_LEVEL_MIN_BLOCKS) k_level(LevelArgs a) {
+// One CTA per SM: the phases are chains of dependent loads, so registers for
+// loads in flight and a barrier over 148 CTAs instead of 296 are worth more
+// than a second CTA, which left 64 registers a thread and spills.  Refinement
+// of a million-vertex mesh (k = 64) 1.24 -> 1.17 ms, the 27-point grid 17.4 ->
+// 15.6 ms, a 4M circuit (k = 256) 76 -> 64 ms.
+__global__ void __launch_bounds__(kLevelThreads, 1) k_level(LevelArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   u64* s_sort = reinterpret_cast<u64*>(smem_raw);                  // kSortMax u64
   i32* greedy = reinterpret_cast<i32*>(smem_raw + kSortMax * 8);   // kGreedyWords
