@@ -225,17 +225,6 @@ __device__ __forceinline__ void warp_append(bool pred, i32 val, i32* list, i32* 
   base = __shfl_sync(kFullMask, base, leader);
   if (pred) list[base + __popc(mask & ((1u << lane) - 1))] = val;
 }
-__device__ __forceinline__ void warp_append64(bool pred, u64 val, u64* list, i32* counter) {
-  const u32 mask = __ballot_sync(kFullMask, pred);
-  if (!mask) return;
-  const int lane = threadIdx.x & 31;
-  const int leader = __ffs(mask) - 1;
-  i32 base = 0;
-  if (lane == leader) base = atomicAdd(counter, __popc(mask));
-  base = __shfl_sync(kFullMask, base, leader);
-  if (pred) list[base + __popc(mask & ((1u << lane) - 1))] = val;
-}
-
 __device__ __forceinline__ u64 globaltimer_ns() {
   u64 t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -385,6 +374,145 @@ __device__ void ph_lists(const LevelArgs& a) {
   }
 }
 
+// Long rows.  A row of more than 64 entries is walked kRowU entries a lane at
+// a time, their ids and weights, then their parts, loaded together: the walk
+// waits for memory once per 256 entries instead of per 32.  It leaves the
+// row's connection weights in acc and the neighbouring parts in a bit set
+// (a part may be joined by zero weights alone), so that the best part is
+// found, and acc cleared, by one walk over the parts instead of two more over
+// the row -- unless there are far more parts than entries (long_by_parts).
+// Rows of more than kRowCta entries are walked by the whole CTA (2048: a walk
+// of all warps costs four barriers, and rows near 1000 entries are plenty on
+// dense levels; 1024 took 39 us where 2048 takes 27).  The rounds' gain
+// updates of a 4M-vertex circuit graph (hubs of 10k entries, coarse rows of
+// about 1100) at k = 256 took 19 to 112 us a round by level, now 7 to 38; its
+// balance rounds 365 us, now 92.
+constexpr i32 kRowU = 8;
+constexpr i32 kRowCta = 2048;
+constexpr i32 kRowList = 64;   // rows a CTA keeps for the walk of all its warps
+__device__ __forceinline__ bool long_by_parts(const LevelArgs& a, i32 len) { return len > 64 && a.kacc <= 4 * len; }
+__device__ __forceinline__ i32 part_words(i32 k) { return (k + 31) >> 5; }
+
+__device__ __forceinline__ void row_connections(const LevelArgs& a, u32* accb, u32* bits, i32 pb, i32 beg, i32 end,
+                                                i32 first, i32 step) {
+  for (i32 e0 = beg + first; e0 < end; e0 += step * kRowU) {
+    i32 q[kRowU];
+    u32 w[kRowU];
+#pragma unroll
+    for (i32 x = 0; x < kRowU; ++x) {
+      const i32 e = e0 + x * step;
+      q[x] = e < end ? a.adjncy[e] : -1;
+      w[x] = e < end ? (u32)a.adjwgt[e] : 0u;
+    }
+#pragma unroll
+    for (i32 x = 0; x < kRowU; ++x) q[x] = q[x] >= 0 ? ldc(a.part + q[x]) : -1;
+#pragma unroll
+    for (i32 x = 0; x < kRowU; ++x) {
+      if (q[x] < 0) continue;
+      atomicAdd(&accb[q[x]], w[x]);
+      const i32 ql = q[x] - pb;
+      if (!((bits[ql >> 5] >> (ql & 31)) & 1u)) atomicOr(&bits[ql >> 5], 1u << (ql & 31));
+    }
+  }
+}
+
+// The best part of the gain rule among the marked parts (its key, see
+// ph_update_rows), for parts first, first + step, ...; clears acc.  *others:
+// some marked part is not p.
+__device__ __forceinline__ u64 best_marked_part(const LevelArgs& a, u32* accb, const u32* bits, i32 pb, i32 p, u32 id,
+                                                i32 first, i32 step, bool* others) {
+  u64 best = 0;
+  for (i32 ql = first; ql < a.kacc; ql += step) {
+    if (!((bits[ql >> 5] >> (ql & 31)) & 1u)) continue;
+    const i32 q = pb + ql;
+    if (q != p) {
+      *others = true;
+      const u64 key = ((u64)(accb[q] - id) << 32) | (u32)(~(u32)q);
+      best = best > key ? best : key;
+      accb[q] = 0;   // (acc of p is read as id by every lane before: the caller clears it)
+    }
+  }
+  return best;
+}
+
+__device__ __forceinline__ void write_gain(const LevelArgs& a, UStage& S, i32 v, i32 p, i32 wasP, bool b, u64 best) {
+  u32 g = 0, q_best = (u32)p;
+  const u32 gb = (u32)(best >> 32);
+  if (b && gb > 0) { g = gb; q_best = ~(u32)best; }
+  a.updflag[v] = 0;
+  a.bnd[v] = b ? 1 : 0;
+  a.gain[v] = (i32)g;
+  a.target[v] = (i32)q_best;
+  if ((i32)g > 0 && !wasP) {
+    a.inP[v] = 1;
+    ustage_push(S, v, a.P0, &a.st->pcount[0]);
+  }
+}
+
+// One long row by a warp.
+__device__ __forceinline__ void update_long_row(const LevelArgs& a, u32* acc, u32* bits, UStage& S, i32 v, i32 p,
+                                                i32 wasP, i32 pb, i32 beg, i32 end) {
+  const int lane = threadIdx.x & 31;
+  u32* accb = acc - pb;
+  for (i32 x = lane; x < part_words(a.kacc); x += 32) bits[x] = 0;
+  __syncwarp();
+  row_connections(a, accb, bits, pb, beg, end, lane, 32);
+  __syncwarp();
+  const u32 id = accb[p];
+  __syncwarp();
+  bool others = false;
+  u64 best = best_marked_part(a, accb, bits, pb, p, id, lane, 32, &others);
+  best = warp_max_key(best);
+  const bool b = __any_sync(kFullMask, others);
+  if (lane == 0) {
+    accb[p] = 0;
+    write_gain(a, S, v, p, wasP, b, best);
+  }
+  __syncwarp();
+}
+
+// The CTA's listed rows, each by all its warps (block-uniform; acc row 0 and
+// the bits are free and zero / to be cleared here).
+struct RowList {
+  i32 v[kRowList];
+  i32 n;
+  u64 red[kLevelThreads / 32];
+  i32 any;
+};
+__device__ __forceinline__ bool row_list_push(RowList& L, i32 v) {   // one lane; false when full
+  const i32 at = atomicAdd(&L.n, 1);
+  if (at < kRowList) L.v[at] = v;
+  return at < kRowList;
+}
+__device__ void update_listed_rows(const LevelArgs& a, u32* acc, u32* bits, UStage& S, RowList& L) {
+  __syncthreads();
+  const i32 n = L.n < kRowList ? L.n : kRowList;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (i32 x = 0; x < n; ++x) {
+    const i32 v = L.v[x];
+    const i32 p = ldc(a.part + v), pb = part_base_of(a, v);
+    u32* accb = acc - pb;
+    for (i32 q = threadIdx.x; q < part_words(a.kacc); q += blockDim.x) bits[q] = 0;
+    if (threadIdx.x == 0) L.any = 0;
+    __syncthreads();
+    row_connections(a, accb, bits, pb, a.xadj[v], a.xadj[v + 1], (i32)threadIdx.x, (i32)blockDim.x);
+    __syncthreads();
+    const u32 id = accb[p];
+    bool others = false;
+    u64 best = best_marked_part(a, accb, bits, pb, p, id, (i32)threadIdx.x, (i32)blockDim.x, &others);
+    best = warp_max_key(best);
+    if (lane == 0) L.red[wid] = best;
+    if (others) L.any = 1;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < (int)(blockDim.x >> 5); ++w) best = L.red[w] > best ? L.red[w] : best;
+      accb[p] = 0;
+      write_gain(a, S, v, p, ldc(a.inP + v), L.any != 0, best);
+    }
+    __syncthreads();
+  }
+}
+
 // Gain update (uncoarsen.hpp:175-237, update_vertex_info + calculate_gain).
 // One warp per vertex of U, per-part connection weights in a per-warp shared
 // row of k words (only touched entries are cleared afterwards).  The best part
@@ -394,23 +522,40 @@ __device__ void ph_lists(const LevelArgs& a) {
 // Vertices whose new gain is positive join P.
 // `count`: add the row lengths read to the level's entry counter (the update
 // passes of the rounds; the first pass of a level is counted as a full pass).
-__device__ void ph_update_rows(const LevelArgs& a, u32* acc_all, bool count, UStage& S, i32 nU_known) {
+__device__ void ph_update_rows(const LevelArgs& a, u32* acc_all, u32* bits_all, bool count, UStage& S, RowList& L,
+                               i32 nU_known) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (wid >= a.acc_warps) return;
   u32* acc = acc_all + (size_t)wid * a.kacc;
+  u32* bits = bits_all + (size_t)wid * part_words(a.kacc);
   RoundState* st = a.st;
   const i32 nU = nU_known >= 0 ? nU_known : ldc(&st->ucount);
   i32* Pout = a.P0;          // P is never compacted within a level: entries whose
   i32* pcount = &st->pcount[0];   // gain dropped stay and are skipped by gain
   const i64 nw = (i64)gridDim.x * a.acc_warps;
   unsigned long long rows = 0;
-  for (i64 i = (i64)blockIdx.x * a.acc_warps + wid; i < nU; i += nw) {
-    const i32 v = ldc(a.U + i);
-    const i32 p = ldc(a.part + v);
-    const i32 wasP = ldc(a.inP + v);   // U holds v once: no other warp writes inP[v] in this phase
+  // The next vertex's id is loaded two rows ahead and its header one row
+  // ahead, beside the current row's chain (U holds a vertex once: no other
+  // warp writes its inP in this phase).
+  i64 i = (i64)blockIdx.x * a.acc_warps + wid;
+  i32 vn = i < nU ? ldc(a.U + i) : 0, vnn = i + nw < nU ? ldc(a.U + i + nw) : 0;
+  i32 pn = 0, wn = 0, bn = 0, en = 0;
+  auto header = [&](bool on) {
+    if (on) {
+      pn = ldc(a.part + vn);
+      wn = ldc(a.inP + vn);
+      bn = a.xadj[vn];
+      en = a.xadj[vn + 1];
+    }
+  };
+  header(i < nU);
+  for (; i < nU; i += nw) {
+    const i32 v = vn, p = pn, wasP = wn, beg = bn, end = en;
+    vn = vnn;
+    if (i + 2 * nw < nU) vnn = ldc(a.U + i + 2 * nw);
+    header(i + nw < nU);
     const i32 pb = part_base_of(a, v);   // rows are indexed by the graph's own part ids
     u32* accb = acc - pb;
-    const i32 beg = a.xadj[v], end = a.xadj[v + 1];
     rows += (unsigned long long)(end - beg);
     u32 g = 0, q_best = (u32)p;
     bool b;
@@ -450,6 +595,15 @@ __device__ void ph_update_rows(const LevelArgs& a, u32* acc_all, bool count, USt
       if (h0) accb[q0] = 0;
       if (h1) accb[q1] = 0;
       __syncwarp();
+      continue;
+    }
+    if (long_by_parts(a, end - beg)) {   // warp-uniform
+      bool listed = false;
+      if (end - beg > kRowCta) {
+        if (lane == 0) listed = row_list_push(L, v);
+        listed = __shfl_sync(kFullMask, (int)listed, 0) != 0;
+      }
+      if (!listed) update_long_row(a, acc, bits, S, v, p, wasP, pb, beg, end);
       continue;
     }
     bool bl = false;
@@ -495,10 +649,15 @@ __device__ void ph_update_rows(const LevelArgs& a, u32* acc_all, bool count, USt
 // global atomic; every thread of the CTA calls this.
 // Returns (thread 0) the CTA's appends to P.  nU_known: the length of U when
 // the caller has it (from grid_barrier_count), else -1.
-__device__ u32 ph_update(const LevelArgs& a, u32* acc_all, bool count, UStage& S, i32 nU_known = -1) {
-  if (threadIdx.x == 0) S.cnt = 0;
+__device__ u32 ph_update(const LevelArgs& a, u32* acc_all, u32* bits_all, bool count, UStage& S, RowList& L,
+                         i32 nU_known = -1) {
+  if (threadIdx.x == 0) {
+    S.cnt = 0;
+    L.n = 0;
+  }
   __syncthreads();
-  ph_update_rows(a, acc_all, count, S, nU_known);
+  ph_update_rows(a, acc_all, bits_all, count, S, L, nU_known);
+  update_listed_rows(a, acc_all, bits_all, S, L);
   ustage_flush(S, a.P0, &a.st->pcount[0]);
   __syncthreads();
   return (u32)S.cnt;
@@ -511,14 +670,18 @@ __device__ u32 ph_update(const LevelArgs& a, u32* acc_all, bool count, UStage& S
 // level kernel's sort and greedy buffers (free during an update phase); the
 // rows are zeroed here and every vertex clears the entries it touched.
 template <int G>
-__device__ void ph_update_first_groups(const LevelArgs& a, u32* rows, UStage& S) {
+__device__ void ph_update_first_groups(const LevelArgs& a, u32* rows, u32* acc_all, u32* bits_all, UStage& S,
+                                       RowList& L) {
   constexpr int kGpw = 32 / G;   // groups per warp
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int sub = lane & (G - 1), grp = lane / G;
   const u32 gmask = (G == 32 ? kFullMask : ((1u << G) - 1u)) << (grp * G);
   const i32 ngrp = (i32)(blockDim.x / G);
   for (i32 q = threadIdx.x; q < ngrp * a.kacc; q += blockDim.x) rows[q] = 0;
-  if (threadIdx.x == 0) S.cnt = 0;
+  if (threadIdx.x == 0) {
+    S.cnt = 0;
+    L.n = 0;
+  }
   __syncthreads();
   u32* acc = rows + (size_t)(wid * kGpw + grp) * a.kacc;
   RoundState* st = a.st;
@@ -526,17 +689,54 @@ __device__ void ph_update_first_groups(const LevelArgs& a, u32* rows, UStage& S)
   i32* Pout = a.P0;
   i32* pcount = &st->pcount[0];
   const i64 step = (i64)gridDim.x * ngrp;
-  // warp-uniform trip count: a warp's groups take vertices base .. base + kGpw - 1
-  for (i64 base = ((i64)blockIdx.x * blockDim.x + (threadIdx.x & ~31)) / G; base < nU; base += step) {
+  // warp-uniform trip count: a warp's groups take vertices base .. base + kGpw - 1;
+  // ids are loaded two vertices ahead and headers one, as in ph_update_rows
+  const i64 base0 = ((i64)blockIdx.x * blockDim.x + (threadIdx.x & ~31)) / G;
+  i32 vn = base0 + grp < nU ? ldc(a.U + base0 + grp) : 0;
+  i32 vnn = base0 + step + grp < nU ? ldc(a.U + base0 + step + grp) : 0;
+  i32 pn = 0, wn = 1, bn = 0, en = 0;
+  auto header = [&](bool on) {
+    pn = 0;
+    wn = 1;
+    bn = en = 0;
+    if (on) {
+      pn = ldc(a.part + vn);
+      wn = ldc(a.inP + vn);
+      bn = a.xadj[vn];
+      en = a.xadj[vn + 1];
+    }
+  };
+  header(base0 + grp < nU);
+  for (i64 base = base0; base < nU; base += step) {
     const i64 i = base + grp;
-    const bool act = i < nU;
-    i32 v = 0, p = 0, wasP = 1, beg = 0, end = 0;
-    if (act) {
-      v = ldc(a.U + i);
-      p = ldc(a.part + v);
-      wasP = ldc(a.inP + v);
-      beg = a.xadj[v];
-      end = a.xadj[v + 1];
+    bool act = i < nU;
+    const i32 v = vn, p = pn, wasP = wn, beg = bn;
+    i32 end = en;
+    vn = vnn;
+    if (i + 2 * step < nU) vnn = ldc(a.U + i + 2 * step);
+    header(i + step < nU);
+    // a long row would hold its few lanes for thousands of loads: the warp
+    // takes it, or the CTA after the pass
+    u32 lng = __ballot_sync(kFullMask, act && sub == 0 && long_by_parts(a, end - beg));
+    if (lng) {
+      if ((lng >> (grp * G)) & 1u) act = false;   // (its entries below are none)
+      for (u32 t = lng; t; t &= t - 1) {
+        const int src = __ffs(t) - 1;
+        const i32 lv = __shfl_sync(kFullMask, v, src), lp = __shfl_sync(kFullMask, p, src);
+        const i32 lw = __shfl_sync(kFullMask, wasP, src);
+        const i32 lb = __shfl_sync(kFullMask, beg, src), le = __shfl_sync(kFullMask, end, src);
+        bool listed = false;
+        if (le - lb > kRowCta || wid >= a.acc_warps) {
+          if (lane == 0) listed = row_list_push(L, lv);
+          listed = __shfl_sync(kFullMask, (int)listed, 0) != 0;
+        }
+        if (!listed && wid < a.acc_warps)
+          update_long_row(a, acc_all + (size_t)wid * a.kacc, bits_all + (size_t)wid * part_words(a.kacc), S, lv, lp, lw,
+                          part_base_of(a, lv), lb, le);
+        else if (!listed && ((t >> src) & 1u) && grp == src / G)
+          act = true;   // no acc row and a full list: the group takes it after all
+      }
+      if (!act) end = beg;
     }
     u32* accb = acc - (act ? part_base_of(a, v) : 0);   // rows are indexed by the graph's own part ids
     // entries sub and sub + G keep their part ids in registers; longer rows reload
@@ -593,15 +793,16 @@ __device__ void ph_update_first_groups(const LevelArgs& a, u32* rows, UStage& S)
     for (i32 e = e1 + G; e < end; e += G) accb[ldc(a.part + a.adjncy[e])] = 0;
     __syncwarp();
   }
+  update_listed_rows(a, acc_all, bits_all, S, L);
   ustage_flush(S, a.P0, &a.st->pcount[0]);
   __syncthreads();
 }
 
 // The first gain pass: groups of upd_lanes lanes per vertex, or a warp.
-__device__ void ph_update_first(const LevelArgs& a, u32* acc_all, u32* rows, UStage& S) {
-  if (a.upd_lanes == 8) ph_update_first_groups<8>(a, rows, S);
-  else if (a.upd_lanes == 16) ph_update_first_groups<16>(a, rows, S);
-  else ph_update(a, acc_all, false, S);
+__device__ void ph_update_first(const LevelArgs& a, u32* acc_all, u32* bits_all, u32* rows, UStage& S, RowList& L) {
+  if (a.upd_lanes == 8) ph_update_first_groups<8>(a, rows, acc_all, bits_all, S, L);
+  else if (a.upd_lanes == 16) ph_update_first_groups<16>(a, rows, acc_all, bits_all, S, L);
+  else ph_update(a, acc_all, bits_all, false, S, L);
 }
 
 
@@ -665,12 +866,33 @@ __device__ u32 ph_candidates(const LevelArgs& a, i32* s_cnt, i32* s_base, u32* s
       const i32 cv = __shfl_sync(kFullMask, v, src);
       const i32 beg = __shfl_sync(kFullMask, xb, src), end = __shfl_sync(kFullMask, xe, src);
       bool blocked = false;
-      for (i32 e = beg + lane; e < end && !blocked; e += 32) {
-        const i32 u = a.adjncy[e];
-        if (u < cv) {
-          const i32 gu = ldc(a.gain + u), tu = ldc(a.target + u);   // issued together
-          const u32 vu = (u32)a.vwgt[u];
-          if (gu > 0) blocked = valid_move(pw_of(tu), vu, maxw_of(a, tu));
+      if (end - beg <= 64) {   // warp-uniform
+        for (i32 e = beg + lane; e < end && !blocked; e += 32) {
+          const i32 u = a.adjncy[e];
+          if (u < cv) {
+            const i32 gu = ldc(a.gain + u), tu = ldc(a.target + u);   // issued together
+            const u32 vu = (u32)a.vwgt[u];
+            if (gu > 0) blocked = valid_move(pw_of(tu), vu, maxw_of(a, tu));
+          }
+        }
+      } else {   // long rows: kRowU entries a lane together, until a lane is blocked
+        bool any = false;
+        for (i32 b0 = beg; b0 < end && !any; b0 += 32 * kRowU) {
+          i32 u[kRowU], gu[kRowU];
+#pragma unroll
+          for (i32 x = 0; x < kRowU; ++x) {
+            const i32 e = b0 + 32 * x + lane;
+            u[x] = e < end ? a.adjncy[e] : INT_MAX;
+          }
+#pragma unroll
+          for (i32 x = 0; x < kRowU; ++x) gu[x] = u[x] < cv ? ldc(a.gain + u[x]) : 0;
+#pragma unroll
+          for (i32 x = 0; x < kRowU; ++x)
+            if (gu[x] > 0 && !blocked) {
+              const i32 tu = ldc(a.target + u[x]);
+              blocked = valid_move(pw_of(tu), (u32)a.vwgt[u[x]], maxw_of(a, tu));
+            }
+          any = __any_sync(kFullMask, blocked);
         }
       }
       const bool any_blocked = __any_sync(kFullMask, blocked);
@@ -1581,6 +1803,23 @@ __device__ void ph_select_batch(const LevelArgs& a, u64* s, i32* greedy, u64* s_
 }
 
 
+// The neighbours in a row join U unless they are in it (a warp; four entries a
+// lane together).
+__device__ __forceinline__ void mark_row(const LevelArgs& a, UStage& S, i32 beg, i32 end) {
+  const int lane = threadIdx.x & 31;
+  constexpr i32 kU = 4;
+  for (i32 e0 = beg + lane; e0 < end; e0 += 32 * kU) {
+    i32 u[kU], was[kU];
+#pragma unroll
+    for (i32 x = 0; x < kU; ++x) u[x] = e0 + 32 * x < end ? a.adjncy[e0 + 32 * x] : -1;
+#pragma unroll
+    for (i32 x = 0; x < kU; ++x) was[x] = u[x] >= 0 ? atomicExch(&a.updflag[u[x]], 1) : 1;
+#pragma unroll
+    for (i32 x = 0; x < kU; ++x)
+      if (was[x] == 0) ustage_push(S, u[x], a.U, &a.st->ucount);
+  }
+}
+
 // One move, by one warp: v goes to its target; v and its neighbours are
 // flagged for the gain update and appended to U (uncoarsen.hpp:290-323).
 // The part-weight change goes to pwc: pw itself, or the round's delta array
@@ -1599,10 +1838,7 @@ __device__ __forceinline__ void apply_move(const LevelArgs& a, UStage& S, u64 ke
     atomicAdd(s_gsum, (unsigned long long)(i64)key_gain(key));
     if (atomicExch(&a.updflag[v], 1) == 0) ustage_push(S, v, a.U, &a.st->ucount);
   }
-  for (i32 e = beg + lane; e < end; e += 32) {
-    const i32 u = a.adjncy[e];
-    if (atomicExch(&a.updflag[u], 1) == 0) ustage_push(S, u, a.U, &a.st->ucount);
-  }
+  mark_row(a, S, beg, end);
 }
 
 // Batched level: apply every graph's kept moves, top[0..mcount).  One warp
@@ -2055,10 +2291,11 @@ __device__ void ph_bal_filter(const LevelArgs& a) {
   }
 }
 
-__device__ void ph_bal_eval(const LevelArgs& a, u32* acc_all) {
+__device__ void ph_bal_eval(const LevelArgs& a, u32* acc_all, u32* bits_all) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (wid >= a.acc_warps) return;
   u32* acc = acc_all + (size_t)wid * a.kacc;
+  u32* bits = bits_all + (size_t)wid * part_words(a.kacc);
   RoundState* st = a.st;
   const u32 ep = ldc(&st->epoch);
   const i32 light_plain = a.batch ? 0 : ldc(&st->light);
@@ -2072,16 +2309,28 @@ __device__ void ph_bal_eval(const LevelArgs& a, u32* acc_all) {
     u32* accb = acc - pb;   // rows are indexed by the graph's own part ids
     const i32 light = a.batch ? ldc(a.glight + __ldg(a.gid + v)) : light_plain;
     const i32 beg = a.xadj[v], end = a.xadj[v + 1];
-    for (i32 e = beg + lane; e < end; e += 32) atomicAdd(&accb[ldc(a.part + a.adjncy[e])], (u32)a.adjwgt[e]);
+    const bool by_parts = long_by_parts(a, end - beg);   // warp-uniform
+    if (by_parts) {
+      for (i32 x = lane; x < part_words(a.kacc); x += 32) bits[x] = 0;
+      __syncwarp();
+      row_connections(a, accb, bits, pb, beg, end, lane, 32);
+    } else {
+      for (i32 e = beg + lane; e < end; e += 32) atomicAdd(&accb[ldc(a.part + a.adjncy[e])], (u32)a.adjwgt[e]);
+    }
     __syncwarp();
     const u32 id = accb[p];
     u64 best = 0;
-    for (i32 e = beg + lane; e < end; e += 32) {
-      const i32 q = ldc(a.part + a.adjncy[e]);
-      if (q == p || over_cap(ldc(a.pw + q) + w, bcap_of(a, q))) continue;
+    auto consider = [&](i32 q) {
+      if (q == p || over_cap(ldc(a.pw + q) + w, bcap_of(a, q))) return;
       const i32 g = (i32)(accb[q] - id);
       const u64 key = (1ull << 63) | ((u64)((u32)g ^ 0x80000000u) << 31) | (u64)(0x7fffffffu - (u32)q);
       best = best > key ? best : key;
+    };
+    if (by_parts) {
+      for (i32 ql = lane; ql < a.kacc; ql += 32)
+        if ((bits[ql >> 5] >> (ql & 31)) & 1u) consider(pb + ql);
+    } else {
+      for (i32 e = beg + lane; e < end; e += 32) consider(ldc(a.part + a.adjncy[e]));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -2102,37 +2351,49 @@ __device__ void ph_bal_eval(const LevelArgs& a, u32* acc_all) {
       a.bgain[v] = g_best;
     }
     __syncwarp();
-    for (i32 e = beg + lane; e < end; e += 32) accb[ldc(a.part + a.adjncy[e])] = 0;
+    if (by_parts)
+      for (i32 ql = lane; ql < a.kacc; ql += 32) acc[ql] = 0;
+    else
+      for (i32 e = beg + lane; e < end; e += 32) accb[ldc(a.part + a.adjncy[e])] = 0;
     __syncwarp();
   }
 }
 
+// One warp per listed vertex (a lane per vertex walked a coarse row of
+// thousands of entries alone: 135 us a round on a 4M-vertex circuit graph's
+// coarsest balance level).
 __device__ void ph_bal_emit(const LevelArgs& a) {
   RoundState* st = a.st;
   const int lane = threadIdx.x & 31;
   const i32 nl = ldc(&st->lcount);
   const u32 ep = ldc(&st->epoch);
-  const i64 stride = (i64)gridDim.x * blockDim.x;
-  for (i64 base = (i64)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < nl; base += stride) {
-    const i64 i = base + lane;
-    bool emit = false;
-    i32 v = 0, g = 0;
-    if (i < nl) {
-      v = ldc(a.blist + i);
-      emit = ldc(a.bmark + v) == ep;
-      g = emit ? ldc(a.bgain + v) : 0;
-      for (i32 e = a.xadj[v]; emit && e < a.xadj[v + 1]; ++e) {
-        const i32 u = a.adjncy[e];
-        if (u < v && ldc(a.bmark + u) == ep) { emit = false; break; }
+  const i64 nw = ((i64)gridDim.x * blockDim.x) >> 5;
+  for (i64 i = ((i64)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nl; i += nw) {
+    const i32 v = ldc(a.blist + i);
+    if (ldc(a.bmark + v) != ep) continue;   // warp-uniform
+    const i32 g = ldc(a.bgain + v);
+    const i32 beg = a.xadj[v], end = a.xadj[v + 1];
+    bool emit = true;
+    constexpr i32 kU = 4;
+    for (i32 b0 = beg; b0 < end && emit; b0 += 32 * kU) {
+      i32 u[kU];
+      bool yields = false;
+#pragma unroll
+      for (i32 x = 0; x < kU; ++x) {
+        const i32 e = b0 + 32 * x + lane;
+        u[x] = e < end ? a.adjncy[e] : INT_MAX;
       }
+#pragma unroll
+      for (i32 x = 0; x < kU; ++x) yields |= u[x] < v && ldc(a.bmark + u[x]) == ep;
+      emit = !__any_sync(kFullMask, yields);
     }
-    if (a.batch) {   // graph buckets, as in ph_candidates
-      if (emit) {
+    if (emit && lane == 0) {
+      if (a.batch) {   // graph buckets, as in ph_candidates
         const i32 gv = __ldg(a.gid + v);
         a.cands[__ldg(a.gvbase + gv) + atomicAdd(a.gcc + gv, 1)] = move_key(g, v);
+      } else {
+        a.cands[atomicAdd(&st->ccount, 1)] = move_key(g, v);
       }
-    } else {
-      warp_append64(emit, move_key(g, v), a.cands, &st->ccount);
     }
   }
 }
@@ -2159,11 +2420,7 @@ __device__ void ph_apply_balance(const LevelArgs& a, UStage& S) {
       a.part[v] = d;
       if (atomicExch(&a.updflag[v], 1) == 0) ustage_push(S, v, a.U, &st->ucount);
     }
-    const i32 beg = a.xadj[v], end = a.xadj[v + 1];
-    for (i32 e = beg + lane; e < end; e += 32) {
-      const i32 u = a.adjncy[e];
-      if (atomicExch(&a.updflag[u], 1) == 0) ustage_push(S, u, a.U, &st->ucount);
-    }
+    mark_row(a, S, a.xadj[v], a.xadj[v + 1]);
   }
   ustage_flush(S, a.U, &st->ucount);
 }
@@ -2188,6 +2445,8 @@ __global__ void __launch_bounds__(kLevelThreads, 1) k_level(LevelArgs a) {
   __shared__ i32 s_cnt, s_base;
   __shared__ UStage s_ustage;
   __shared__ RankedMoves s_ranked;
+  __shared__ RowList s_rows;
+  u32* bits_all = reinterpret_cast<u32*>(s_keep);   // the gain updates' part sets (no moves are kept then)
   if (threadIdx.x == 0)
     s_ranked = a.batch ? RankedMoves{nullptr, nullptr, nullptr, a.part, a.target, a.vwgt, a.pw, a.pmaxw, 0.f}
                        : RankedMoves{a.cinfo, a.cw, a.risk, nullptr, nullptr, nullptr, a.pw, nullptr, a.maxw};
@@ -2218,7 +2477,7 @@ __global__ void __launch_bounds__(kLevelThreads, 1) k_level(LevelArgs a) {
     if (!grid_barrier(a.bar, a.err, &s_flag)) return;
     trace_mark(a, 2);
   }
-  if (a.flags & LF_UPDATE) ph_update_first(a, acc_all, reinterpret_cast<u32*>(smem_raw), s_ustage);
+  if (a.flags & LF_UPDATE) ph_update_first(a, acc_all, bits_all, reinterpret_cast<u32*>(smem_raw), s_ustage, s_rows);
   if (a.flags & LF_BALANCE) {
     if (a.batch) ph_bal_prep_batch(a, s_tmp, fr);
     else ph_bal_prep(a, s_tmp);
@@ -2239,7 +2498,7 @@ __global__ void __launch_bounds__(kLevelThreads, 1) k_level(LevelArgs a) {
       ph_bal_filter(a);
       if (!grid_barrier(a.bar, a.err, &s_flag)) return;
       trace_mark(a, 9);
-      ph_bal_eval(a, acc_all);
+      ph_bal_eval(a, acc_all, bits_all);
       if (!grid_barrier(a.bar, a.err, &s_flag)) return;
       trace_mark(a, 10);
       ph_bal_emit(a);
@@ -2254,7 +2513,7 @@ __global__ void __launch_bounds__(kLevelThreads, 1) k_level(LevelArgs a) {
       ph_apply_balance(a, s_ustage);
       if (!grid_barrier(a.bar, a.err, &s_flag)) return;
       trace_mark(a, 14);
-      ph_update(a, acc_all, true, s_ustage);
+      ph_update(a, acc_all, bits_all, true, s_ustage, s_rows);
       if (a.batch) ph_bal_prep_batch(a, s_tmp, fr);
       else ph_bal_prep(a, s_tmp);
       if (!grid_barrier(a.bar, a.err, &s_flag)) return;
@@ -2288,7 +2547,7 @@ __global__ void __launch_bounds__(kLevelThreads, 1) k_level(LevelArgs a) {
         ph_apply_refine(a, s_ustage);
         if (!grid_barrier(a.bar, a.err, &s_flag)) return;
         trace_mark(a, 23);
-        ph_update(a, acc_all, true, s_ustage);
+        ph_update(a, acc_all, bits_all, true, s_ustage, s_rows);
         if (!grid_barrier(a.bar, a.err, &s_flag)) return;
         trace_mark(a, 24);
         continue;
@@ -2301,7 +2560,7 @@ __global__ void __launch_bounds__(kLevelThreads, 1) k_level(LevelArgs a) {
       const u32 my_u = ph_refine_apply(a, s_sort, greedy, s_keep, s_warp, s_tmp, &s_ranked, s_ustage, nC);
       if (!grid_barrier_count(a.cbar, cbk++, a.err, &s_flag, &s_total, my_u, &nU)) return;
       trace_mark(a, 23);
-      const u32 my_p = ph_update(a, acc_all, true, s_ustage, nU);
+      const u32 my_p = ph_update(a, acc_all, bits_all, true, s_ustage, s_rows, nU);
       ph_fold(a);
       if (!grid_barrier_count(a.cbar, cbk++, a.err, &s_flag, &s_total, my_p, &nPadd)) return;
       nP = nPadd < 0 ? ldc(&st->pcount[0]) : nP + nPadd;
