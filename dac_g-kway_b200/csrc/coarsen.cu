@@ -198,95 +198,175 @@ void run_match(Handle& h, const DevGraph& g, i32* cand, i64 maxdeg) {
 }
 
 // ===========================================================================
-// Union-find label propagation (coarsen.hpp:80-118, loop :461-469), Jacobi
-// schedule, as one persistent cooperative kernel.  Keys are
-// (label << 32 | round of last raise).  Round r reads buffer (r-1)&1 and
-// raises buffer r&1 with atomicMax; that buffer still holds round r-2's keys,
-// which never exceed round r-1's, so max(own key, pushes) is exactly the
-// synchronous update.  chg[r&1] records whether round r raised anything; the
-// grid barrier separates rounds and the loop ends after the first quiet
-// round -- no host round trip per round.
+// Union-find label propagation (coarsen.hpp:80-118, loop :461-469).  Under the
+// Jacobi schedule a vertex ends with the largest id of its component of
+// candidate edges and the round that brought it, which is its hop distance
+// from that vertex; the loop ends with the first quiet round, one after the
+// largest distance.  No rounds are run here:
+//   hook      every vertex starts at the larger end of its edge; the edges to
+//             smaller ends join their roots, the smaller root under the larger
+//             (lock-free, compare-and-swap)
+//   mark      a component has one cycle of candidates (a mutual pair, or a
+//             longer one), so its root walks its candidates once round that
+//             cycle and marks the distances of the vertices it meets: the
+//             steps taken, and on the cycle the shorter way round
+//   walk      every other vertex finds its root, and follows its candidates to
+//             the first marked vertex: all its ways to the root lead there, so
+//             its distance is the steps plus that mark
+// All are chains of dependent loads per vertex that need no barrier between
+// them, at full occupancy.  Raising labels round by round took a grid barrier
+// and n atomics each (12M-vertex road graph, all levels: 2.66 ms, now 0.92; a
+// million-vertex mesh 0.29 ms, now 0.20; the 27-point grid with its 57 rounds
+// 0.54 ms, now 0.30).
 // ===========================================================================
-constexpr int kUfThreads = 512;
-constexpr int kUfIlp = 2;   // vertices per thread whose loads are issued together
+constexpr int kUfSmallThreads = 1024;
+constexpr i32 kUfSmall = 16384;   // levels up to this run on one CTA, in shared memory
+constexpr u32 kUfUnknown = 0xffffffffu;
 
-__global__ void __launch_bounds__(kUfThreads, 3) k_uf_persist(i32 n, const i32* __restrict__ cand, u64* k0, u64* k1,
-                                                          i32* chg, GridBarrier* bar, i32* err, i32* rounds_out,
-                                                          i32 max_rounds) {
-  __shared__ i32 s_flag, s_any;
-  const i64 stride = (i64)gridDim.x * blockDim.x;
-  const i64 t0 = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-  for (i64 v = t0; v < n; v += stride) {
-    const u64 key = (u64)(u32)v << 32;
-    k0[v] = key;
-    k1[v] = key;
+// Words that other threads of the launch write: from shared memory, or L2.
+template <bool kShared, class T>
+__device__ __forceinline__ T uf_ld(const T* p) { return kShared ? *(const volatile T*)p : __ldcg(p); }
+
+template <bool kShared>
+__device__ __forceinline__ i32 uf_find(i32* parent, i32 x) {   // parents only rise: ends at the root
+  i32 p = uf_ld<kShared>(parent + x);
+  while (p != x) {
+    const i32 g = uf_ld<kShared>(parent + p);
+    if (g != p) *(volatile i32*)(parent + x) = g;   // path halving; any ancestor is a valid parent
+    x = p;
+    p = g;
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    chg[0] = 0;
-    chg[1] = 0;
-    chg[2] = 0;
+  return x;
+}
+
+template <bool kShared>
+__device__ __forceinline__ void uf_unite(i32* parent, i32 x, i32 y) {
+  for (;;) {   // a failed swap means a root rose: ends
+    x = uf_find<kShared>(parent, x);
+    y = uf_find<kShared>(parent, y);
+    if (x == y) return;
+    const i32 lo = x < y ? x : y, hi = x < y ? y : x;
+    const i32 old = atomicCAS(&parent[lo], lo, hi);
+    if (old == lo) return;
+    x = hi;
+    y = old;
   }
-  if (!grid_barrier(bar, err, &s_flag)) return;
-  i32 rounds = -1;
-  for (i32 it = 1;; ++it) {
-    if (it > max_rounds) {   // uniform across CTAs
-      if (blockIdx.x == 0 && threadIdx.x == 0) atomicExch(err, 2);
-      return;
-    }
-    const u64* src = (it & 1) ? k0 : k1;   // round it reads buffer (it-1)&1, raises it&1
-    u64* dst = (it & 1) ? k1 : k0;
-    if (threadIdx.x == 0) s_any = 0;
-    __syncthreads();
-    bool diff = false;
-    for (i64 v0 = t0; v0 < n; v0 += stride * kUfIlp) {
-      // kUfIlp vertices at a time: their candidate loads, then their key
-      // gathers, then the raises (one vertex's steps in the same order)
-      i32 c[kUfIlp];
-      u64 kv[kUfIlp], kc[kUfIlp];
-#pragma unroll
-      for (int q = 0; q < kUfIlp; ++q) {
-        const i64 v = v0 + q * stride;
-        c[q] = v < n ? cand[v] : 0;
-      }
-#pragma unroll
-      for (int q = 0; q < kUfIlp; ++q) {
-        const i64 v = v0 + q * stride;
-        if (v < n) {
-          kv[q] = ldcg(src + v);
-          kc[q] = ldcg(src + c[q]);
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < kUfIlp; ++q) {
-        const i64 v = v0 + q * stride;
-        if (v >= n) continue;
-        const u32 a = (u32)(kv[q] >> 32), b = (u32)(kc[q] >> 32);
-        atomicMax((unsigned long long*)&dst[v], (unsigned long long)kv[q]);
-        if (a > b) {
-          atomicMax((unsigned long long*)&dst[c[q]], (unsigned long long)(((u64)a << 32) | (u32)it));
-          diff = true;
-        } else if (a < b) {
-          atomicMax((unsigned long long*)&dst[v], (unsigned long long)(((u64)b << 32) | (u32)it));
-          diff = true;
-        }
-      }
-    }
-    if (diff) s_any = 1;
-    __syncthreads();
-    // change flags rotate over three words: round it raises chg[it % 3], which
-    // every thread reads after this round's barrier; block 0 clears
-    // chg[(it + 1) % 3] now, whose last reads (round it - 2) all happened
-    // before their CTAs arrived at the previous barrier
-    if (threadIdx.x == 0 && s_any) atomicOr(&chg[it % 3], 1);
-    if (blockIdx.x == 0 && threadIdx.x == 0) chg[(it + 1) % 3] = 0;
-    if (!grid_barrier(bar, err, &s_flag)) return;
-    if (ldcg(&chg[it % 3]) == 0) {
-      rounds = it;
+}
+
+// Root r marks the vertices on its walk (only this thread marks its component
+// in this phase; the walk closes after at most the component's vertices).
+template <bool kShared>
+__device__ __forceinline__ void uf_mark_root(const i32* cand, u32* dist, i32 r) {
+  i32 x = r;
+  u32 i = 0;
+  u32 k;   // distance of the vertex where the walk closes
+  for (;;) {
+    *(volatile u32*)(dist + x) = i;
+    const i32 c = cand[x];
+    k = uf_ld<kShared>(dist + c);
+    if (k != kUfUnknown) {
+      x = c;
       break;
     }
+    x = c;
+    ++i;
   }
-  // after the first quiet round both buffers hold the fixed point
-  if (blockIdx.x == 0 && threadIdx.x == 0) *rounds_out = rounds;
+  const u32 L = i + 1 - k;   // cycle length
+  if (L <= 2) return;
+  for (u32 j = 1; j < L; ++j) {
+    x = cand[x];
+    *(volatile u32*)(dist + x) = k + (j < L - j ? j : L - j);
+  }
+}
+
+// Distance of v (see walk above); a vertex that another thread has finished
+// by now ends the walk as well.
+template <bool kShared>
+__device__ __forceinline__ u32 uf_walk(const i32* cand, const u32* dist, i32 v) {
+  u32 steps = 0;
+  i32 x = v;
+  for (;;) {
+    const i32 c = cand[x];   // (issued beside the mark)
+    const u32 d = uf_ld<kShared>(dist + x);
+    if (d != kUfUnknown) return steps + d;
+    x = c;
+    ++steps;
+  }
+}
+
+__device__ __forceinline__ void uf_max_rounds(u32 d, i32* rounds_out) {   // every thread of the CTA
+  const u32 m = __reduce_max_sync(kFull, d);
+  if ((threadIdx.x & 31) == 0 && (i32)m + 1 > *(volatile i32*)rounds_out) atomicMax(rounds_out, (i32)m + 1);
+}
+
+// One CTA, everything in shared memory (a 2048-vertex level 25 us, now 10).
+__global__ void __launch_bounds__(kUfSmallThreads) k_uf_small(i32 n, const i32* __restrict__ cand_in,
+                                                              u64* __restrict__ keys, i32* rounds_out) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  i32* parent = reinterpret_cast<i32*>(smem_raw);      // [n]
+  u32* dist = reinterpret_cast<u32*>(parent + n);      // [n]
+  i32* cand = reinterpret_cast<i32*>(dist + n);        // [n]
+  __shared__ i32 s_rounds;
+  const i32 T = (i32)blockDim.x;
+  for (i32 v = threadIdx.x; v < n; v += T) {
+    const i32 c = cand_in[v];
+    cand[v] = c;
+    parent[v] = c > v ? c : v;
+    dist[v] = kUfUnknown;
+  }
+  if (threadIdx.x == 0) s_rounds = 0;
+  __syncthreads();
+  for (i32 v = threadIdx.x; v < n; v += T)
+    if (cand[v] < v) uf_unite<true>(parent, v, cand[v]);
+  __syncthreads();
+  for (i32 v = threadIdx.x; v < n; v += T)
+    if (parent[v] == v) uf_mark_root<true>(cand, dist, v);
+  __syncthreads();
+  u32 m = 0;
+  for (i32 v = threadIdx.x; v < n; v += T) {
+    const u32 d = uf_walk<true>(cand, dist, v);
+    *(volatile u32*)(dist + v) = d;
+    m = d > m ? d : m;
+    keys[v] = ((u64)(u32)uf_find<true>(parent, v) << 32) | d;
+  }
+  uf_max_rounds(m, &s_rounds);
+  __syncthreads();
+  if (threadIdx.x == 0) *rounds_out = s_rounds;
+}
+
+__global__ void k_uf_init(i32 n, const i32* __restrict__ cand, i32* __restrict__ parent, u32* __restrict__ dist,
+                          i32* rounds_out) {
+  const i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+  if (v == 0) *rounds_out = 0;
+  if (v >= n) return;
+  const i32 c = cand[v];
+  parent[v] = c > (i32)v ? c : (i32)v;
+  dist[v] = kUfUnknown;
+}
+
+__global__ void k_uf_hook(i32 n, const i32* __restrict__ cand, i32* parent) {
+  const i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= n) return;
+  const i32 c = cand[v];
+  if (c < (i32)v) uf_unite<false>(parent, (i32)v, c);
+}
+
+__global__ void k_uf_mark(i32 n, const i32* __restrict__ cand, const i32* __restrict__ parent, u32* dist) {
+  const i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+  if (v < n && parent[v] == (i32)v) uf_mark_root<false>(cand, dist, (i32)v);
+}
+
+__global__ void k_uf_walk(i32 n, const i32* __restrict__ cand, i32* parent, u32* dist, u64* __restrict__ keys,
+                          i32* rounds_out) {
+  const i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+  u32 d = 0;
+  if (v < n) {
+    const i32 r = uf_find<false>(parent, (i32)v);
+    d = uf_walk<false>(cand, dist, (i32)v);
+    *(volatile u32*)(dist + v) = d;
+    keys[v] = ((u64)(u32)r << 32) | d;
+  }
+  uf_max_rounds(d, rounds_out);
 }
 
 // Writes the final keys to keys_out and the reference's round-launch count
@@ -297,19 +377,22 @@ void run_union_find(Handle& h, i32 n, const i32* cand, u64* keys_out, i32* d_rou
     GKW_CUDA(cudaMemcpyAsync(d_rounds, &one, sizeof(i32), cudaMemcpyHostToDevice, h.stream));
     return;
   }
+  if (n <= kUfSmall) {
+    if (!h.capturing)
+      GKW_CUDA(cudaFuncSetAttribute(k_uf_small, cudaFuncAttributeMaxDynamicSharedMemorySize, kUfSmall * 12));
+    launch(k_uf_small, 1, kUfSmallThreads, (size_t)n * 12, h.stream, n, cand, keys_out, d_rounds);
+    GKW_CHECK_LAUNCH();
+    return;
+  }
   Pool::Mark mk = h.scratch.mark();
-  u64* kb = h.scratch.alloc_n<u64>(n);
-  i32* chg = h.scratch.alloc_n<i32>(3);
-  static int bps = 0;   // the same on every device of the process (one B200 model)
-  if (!bps) GKW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_uf_persist, kUfThreads, 0));
-  GKW_REQUIRE(bps >= 1, GKW_E_INTERNAL, "union-find kernel does not fit on an SM");
-  i32 grid = std::min<i32>(h.sm_count * std::min(bps, 4), (i32)ceil_div(n, kUfThreads));
-  grid = coop_grid(h, (const void*)k_uf_persist, grid, kUfThreads, 0);
-  i32 max_rounds = n + 2;
-  GridBarrier* barp = &h.coop->bar;
-  i32* errp = &h.coop->err;
-  void* args[] = {&n, &cand, &keys_out, &kb, &chg, &barp, &errp, &d_rounds, &max_rounds};
-  launch_coop(h, (const void*)k_uf_persist, grid, kUfThreads, 0, args);
+  const u32 nb = ceil_div(n, 256);
+  i32* parent = h.scratch.alloc_n<i32>(n);
+  u32* dist = h.scratch.alloc_n<u32>(n);
+  launch(k_uf_init, nb, 256, 0, h.stream, n, cand, parent, dist, d_rounds);
+  launch(k_uf_hook, nb, 256, 0, h.stream, n, cand, parent);
+  launch(k_uf_mark, nb, 256, 0, h.stream, n, cand, (const i32*)parent, dist);
+  launch(k_uf_walk, nb, 256, 0, h.stream, n, cand, parent, dist, keys_out, d_rounds);
+  GKW_CHECK_LAUNCH();
   h.scratch.release(mk);
 }
 
@@ -1399,7 +1482,7 @@ __global__ void __launch_bounds__(kFusedThreads, 2) k_coarsen_fused(FusedArgs a)
     if (!grid_barrier(a.bar, a.err, &s_flag)) return;
   }
 
-  // ---- union-find rounds (coarsen.hpp:80-118, 461-469), as k_uf_persist ----
+  // ---- union-find rounds (coarsen.hpp:80-118, 461-469) as label raising per round ----
   {
     i32 rounds = -1;
     for (i32 it = 1;; ++it) {
