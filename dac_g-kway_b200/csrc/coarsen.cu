@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstddef>
+#include <type_traits>
 
 #include "device_util.cuh"
 
@@ -734,9 +735,106 @@ __device__ void warp_bitonic_u64(u64* a, i32 P, int lane) {
   }
 }
 
-template <int WCAP, int WARPS>
+// Merge of one coarse row whose kept entries lie one per lane in a group of G
+// lanes: `key` the coarse id (kEmpty: none), w the weight.  The group sorts
+// (id, lane) -- 32 bits while ids stay below 2^(32 - log2 G), else 64 -- sums
+// each run of equal ids (mod 2^32) and writes the distinct ids in order at o;
+// returns their number.  Whole warps call it together.
+template <int G, class K>
+__device__ __forceinline__ i32 merge_lanes(u32 key, u32 w, i32 o, i32* __restrict__ sadj, i32* __restrict__ swgt) {
+  constexpr int kBits = G == 32 ? 5 : G == 16 ? 4 : 3;
+  const int lane = threadIdx.x & 31, sub = lane & (G - 1), g0 = lane & ~(G - 1);
+  K x = key == kEmpty ? ~(K)0 : ((K)key << kBits) | (K)sub;
+#pragma unroll
+  for (int kk = 2; kk <= G; kk <<= 1) {
+#pragma unroll
+    for (int jj = kk >> 1; jj > 0; jj >>= 1) {
+      const K y = __shfl_xor_sync(kFull, x, jj, G);
+      const bool keep_min = ((sub & kk) == 0) == ((sub & jj) == 0);
+      x = keep_min ? (x < y ? x : y) : (x < y ? y : x);
+    }
+  }
+  const bool on = x != ~(K)0;
+  const u32 id = on ? (u32)(x >> kBits) : kEmpty;
+  const u32 ww = __shfl_sync(kFull, w, (int)(x & (K)(G - 1)), G);
+  const u32 prev = __shfl_up_sync(kFull, id, 1, G), next = __shfl_down_sync(kFull, id, 1, G);
+  const bool head = sub == 0 || prev != id;
+  const bool last = on && (sub == G - 1 || next != id);
+  u32 S = on ? ww : 0u;   // inclusive prefix sum (mod 2^32)
+#pragma unroll
+  for (int d = 1; d < G; d <<= 1) {
+    const u32 y = __shfl_up_sync(kFull, S, d, G);
+    if (sub >= d) S += y;
+  }
+  const u32 gmask = G == 32 ? kFull : ((1u << G) - 1u);
+  const u32 heads = (__ballot_sync(kFull, head) >> g0) & gmask;
+  const u32 lasts = (__ballot_sync(kFull, last) >> g0) & gmask;
+  const int start = 31 - __clz(heads & (0xffffffffu >> (31 - sub)));   // first lane of this lane's run
+  const u32 before = __shfl_sync(kFull, S, start > 0 ? start - 1 : 0, G);
+  if (last) {
+    const i32 at = o + __popc(lasts & ((1u << sub) - 1u));
+    sadj[at] = (i32)id;
+    swgt[at] = (i32)(S - (start > 0 ? before : 0u));
+  }
+  return __popc(lasts);
+}
+
+// Rows of short levels (a road graph's coarse rows have about 7 entries): 16
+// lanes per coarse vertex, two rows a warp.  Rows that do not fit are listed
+// for k_contract_warp.
+constexpr int kContractG = 16;
+template <class K>
+__global__ void __launch_bounds__(256) k_contract_short(
+    const i32* __restrict__ ncp, const i32* __restrict__ xadj, const i32* __restrict__ adjncy,
+    const i32* __restrict__ adjwgt, const i32* __restrict__ cmap, const i32* __restrict__ memtab,
+    const i32* __restrict__ mcnt, i32 cap, const i32* __restrict__ rowlen, const i32* __restrict__ ub,
+    i32* __restrict__ sadj, i32* __restrict__ swgt, i32* __restrict__ cnt, i32* __restrict__ mid,
+    i32* __restrict__ nmid) {
+  constexpr int G = kContractG;
+  const int lane = threadIdx.x & 31, sub = lane & (G - 1);
+  const i32 nc = *ncp;
+  const i64 ng = ((i64)gridDim.x * blockDim.x) / G;
+  for (i64 c0 = ((i64)blockIdx.x * blockDim.x + (threadIdx.x & ~31)) / G; c0 < nc; c0 += ng) {   // warp-uniform
+    const i64 c = c0 + lane / G;
+    const bool on = c < nc;
+    const i32 L = on ? rowlen[c] : 0, nm = on ? mcnt[c] : 0, o = on ? ub[c] : 0;
+    const bool fits = L <= G && nm <= G;
+    i32 mbeg = 0, mlen = 0;
+    if (fits && sub < nm) {
+      const i32 mv = memtab[c * cap + sub];
+      mbeg = xadj[mv];
+      mlen = xadj[mv + 1] - mbeg;
+    }
+    i32 incl = mlen;
+#pragma unroll
+    for (int d = 1; d < G; d <<= 1) {
+      const i32 y = __shfl_up_sync(kFull, incl, d, G);
+      if (sub >= d) incl += y;
+    }
+    const i32 shift = mbeg - (incl - mlen);
+    i32 jm = 0;   // members whose rows end at or before this lane's entry
+    const i32 nmx = (i32)__reduce_max_sync(kFull, (u32)(fits ? nm : 0));
+    for (i32 j = 0; j < nmx; ++j) jm += sub >= __shfl_sync(kFull, incl, j, G) && j < nm;
+    const i32 pos = __shfl_sync(kFull, shift, jm & (G - 1), G) + sub;
+    u32 key = kEmpty, w = 0;
+    if (fits && sub < L) {
+      key = (u32)cmap[adjncy[pos]];
+      w = (u32)adjwgt[pos];
+      if (key == (u32)c) key = kEmpty;
+    }
+    const i32 u = merge_lanes<G, K>(key, w, o, sadj, swgt);
+    if (on && sub == 0) {
+      if (fits) cnt[c] = u;
+      else mid[atomicAdd(nmid, 1)] = (i32)c;
+    }
+  }
+}
+
+// One warp per coarse row: all of them, or those of a list.
+template <int WCAP, int WARPS, class K>
 __global__ void __launch_bounds__(WARPS * 32) k_contract_warp(
-    const i32* __restrict__ ncp, const i32* __restrict__ xadj, const i32* __restrict__ adjncy, const i32* __restrict__ adjwgt,
+    const i32* __restrict__ ncp, const i32* __restrict__ list, const i32* __restrict__ xadj,
+    const i32* __restrict__ adjncy, const i32* __restrict__ adjwgt,
     const i32* __restrict__ cmap, const i32* __restrict__ memtab, const i32* __restrict__ mcnt, i32 cap,
     const i32* __restrict__ rowlen, const i32* __restrict__ ub, i32* __restrict__ sadj,
     i32* __restrict__ swgt, i32* __restrict__ cnt, i32* __restrict__ heavy, i32* __restrict__ nheavy) {
@@ -744,129 +842,89 @@ __global__ void __launch_bounds__(WARPS * 32) k_contract_warp(
   WarpTable<WCAP>* tabs = reinterpret_cast<WarpTable<WCAP>*>(smem_raw);
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   WarpTable<WCAP>& T = tabs[wid];
-  const i32 nc = *ncp;
+  const i32 nrows = *ncp;   // coarse vertices, or entries of the list
   const i64 nw = (i64)gridDim.x * WARPS;
   // The next coarse vertex's header (row length, member count, this lane's
   // member) is loaded while the current one is contracted: two of the five
   // dependent loads of a coarse row leave the chain.
-  i64 c = (i64)blockIdx.x * WARPS + wid;
-  i32 nL = 0, nnm = 0, nmv = 0;
-  auto header = [&](i64 cc) {
-    if (cc < nc) {
-      nL = rowlen[cc];
-      nnm = mcnt[cc];
-      nmv = lane < cap ? memtab[cc * (i64)cap + lane] : 0;
+  i64 q = (i64)blockIdx.x * WARPS + wid;
+  i32 nL = 0, nnm = 0, nmv = 0, nxc = 0;
+  auto header = [&](i64 qq) {
+    if (qq < nrows) {
+      nxc = list ? list[qq] : (i32)qq;
+      nL = rowlen[nxc];
+      nnm = mcnt[nxc];
+      nmv = lane < cap ? memtab[nxc * (i64)cap + lane] : 0;
     }
   };
-  header(c);
-  for (; c < nc; c += nw) {
-    const i32 L = nL, nm = nnm, mv = nmv;
-    header(c + nw);
+  header(q);
+  for (; q < nrows; q += nw) {
+    const i32 c = nxc, L = nL, nm = nnm, mv = nmv;
+    header(q + nw);
     if (L > WCAP || nm > 32) {
-      if (lane == 0) heavy[atomicAdd(nheavy, 1)] = (i32)c;
+      if (lane == 0) heavy[atomicAdd(nheavy, 1)] = c;
       continue;
     }
-    // lane j < nm: member j's row; exclusive prefix of the row lengths
+    // lane j < nm: member j's row; inclusive prefix of the row lengths
     i32 mbeg = 0, mlen = 0;
     if (lane < nm) {
       mbeg = xadj[mv];
       mlen = xadj[mv + 1] - mbeg;
     }
     const i32 o = ub[c];   // needed only at the writes
-    i32 moff = mlen;
+    i32 incl = mlen;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const i32 y = __shfl_up_sync(kFull, moff, o);
-      if (lane >= o) moff += y;
+    for (int d = 1; d < 32; d <<= 1) {
+      const i32 y = __shfl_up_sync(kFull, incl, d);
+      if (lane >= d) incl += y;
     }
-    moff -= mlen;
+    const i32 shift = mbeg - (incl - mlen);
     // entry i of the concatenated rows -> its CSR position
     auto entry_pos = [&](i32 i) {
-      i32 pos = -1;
-      for (i32 jm = 0; jm < nm; ++jm) {
-        const i32 oj = __shfl_sync(kFull, moff, jm);
-        const i32 lj = __shfl_sync(kFull, mlen, jm);
-        const i32 bj = __shfl_sync(kFull, mbeg, jm);
-        if (i >= oj && i < oj + lj) pos = bj + (i - oj);
-      }
-      return pos;
+      i32 jm = 0;
+      for (i32 j = 0; j < nm; ++j) jm += i >= __shfl_sync(kFull, incl, j);
+      return __shfl_sync(kFull, shift, jm & 31) + i;
     };
     // Rows whose entries other than self loops fit one per lane merge in
     // registers: every row of up to 32 entries, and rows of up to 64 entries
     // with at most 32 left after the self loops (the members' edges to one
     // another) are dropped -- most coarse rows of a mesh.
-    u64 kv = ~0ull;
+    u32 key = kEmpty, w = 0;
     bool in_regs = false;
     if (L <= 32) {
       const i32 pos = entry_pos(lane);
       if (lane < L) {
-        const u32 key = (u32)cmap[adjncy[pos]];
-        if (key != (u32)c) kv = ((u64)key << 32) | (u32)adjwgt[pos];
+        key = (u32)cmap[adjncy[pos]];
+        w = (u32)adjwgt[pos];
+        if (key == (u32)c) key = kEmpty;
       }
       in_regs = true;
     } else if (L <= 64) {
       const i32 p0 = entry_pos(lane), p1 = entry_pos(lane + 32);
-      u64 e0 = ~0ull, e1 = ~0ull;
-      {
-        const u32 k0 = (u32)cmap[adjncy[p0]];
-        if (k0 != (u32)c) e0 = ((u64)k0 << 32) | (u32)adjwgt[p0];
-      }
+      u32 k0 = (u32)cmap[adjncy[p0]], w0 = (u32)adjwgt[p0], k1 = kEmpty, w1 = 0;
       if (lane + 32 < L) {
-        const u32 k1 = (u32)cmap[adjncy[p1]];
-        if (k1 != (u32)c) e1 = ((u64)k1 << 32) | (u32)adjwgt[p1];
+        k1 = (u32)cmap[adjncy[p1]];
+        w1 = (u32)adjwgt[p1];
       }
-      const u32 m0 = __ballot_sync(kFull, e0 != ~0ull), m1 = __ballot_sync(kFull, e1 != ~0ull);
+      if (k0 == (u32)c) k0 = kEmpty;
+      if (k1 == (u32)c) k1 = kEmpty;
+      const u32 m0 = __ballot_sync(kFull, k0 != kEmpty), m1 = __ballot_sync(kFull, k1 != kEmpty);
       const i32 n0 = __popc(m0), tot = n0 + __popc(m1);
       if (tot <= 32) {   // warp-uniform: compact the kept entries to one per lane
         const u32 lt = (1u << lane) - 1u;
-        if (e0 != ~0ull) T.out[__popc(m0 & lt)] = e0;
-        if (e1 != ~0ull) T.out[n0 + __popc(m1 & lt)] = e1;
+        if (k0 != kEmpty) T.out[__popc(m0 & lt)] = ((u64)k0 << 32) | w0;
+        if (k1 != kEmpty) T.out[n0 + __popc(m1 & lt)] = ((u64)k1 << 32) | w1;
         __syncwarp();
-        kv = lane < tot ? T.out[lane] : ~0ull;
+        const u64 kv = lane < tot ? T.out[lane] : ~0ull;
         __syncwarp();
+        key = (u32)(kv >> 32);
+        w = (u32)kv;
         in_regs = true;
       }
     }
     if (in_regs) {
-      // sort (key, w), merge equal keys (self loops are already out)
-#pragma unroll
-      for (int kk = 2; kk <= 32; kk <<= 1) {
-#pragma unroll
-        for (int jj = kk >> 1; jj > 0; jj >>= 1) {
-          const u64 ot = __shfl_xor_sync(kFull, kv, jj);
-          const bool up = (lane & kk) == 0;
-          const bool lower = (lane & jj) == 0;
-          kv = (lower == up) ? umin64(kv, ot) : umax64(kv, ot);
-        }
-      }
-      const u32 key = (u32)(kv >> 32);
-      const u32 w = (u32)kv;
-      const u32 kprev = __shfl_up_sync(kFull, key, 1);
-      const u32 knext = __shfl_down_sync(kFull, key, 1);
-      const bool head = lane == 0 || kprev != key;
-      const bool last = lane == 31 || knext != key;
-      // inclusive prefix sum of w (mod 2^32) and the start lane of each run
-      u32 S = w;
-      i32 start = head ? lane : 0;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const u32 y = __shfl_up_sync(kFull, S, d);
-        const i32 z = __shfl_up_sync(kFull, start, d);
-        if (lane >= d) {
-          S += y;
-          start = start > z ? start : z;
-        }
-      }
-      const u32 before = __shfl_sync(kFull, S, start > 0 ? start - 1 : 0);
-      const u32 total = S - (start > 0 ? before : 0u);
-      const bool valid = last && key != 0xffffffffu;
-      const u32 bal = __ballot_sync(kFull, valid);
-      if (valid) {
-        const i32 at = o + __popc(bal & ((1u << lane) - 1));
-        sadj[at] = (i32)key;
-        swgt[at] = (i32)total;
-      }
-      if (lane == 0) cnt[c] = __popc(bal);
+      const i32 u = merge_lanes<32, K>(key, w, o, sadj, swgt);
+      if (lane == 0) cnt[c] = u;
       continue;
     }
     u32 hsz = 64;
@@ -928,6 +986,122 @@ __global__ void __launch_bounds__(WARPS * 32) k_contract_warp(
   }
 }
 
+// Heavy rows (longer than the warp tables) by direct accumulation: one CTA per
+// row, a weight per coarse id in shared memory (kDenseIds ids at a time, a
+// window of the id range) and a bit per id that was met, whose order is the
+// row's -- no hashing, no sort.  It takes every heavy row of levels with at
+// most kDenseIds coarse vertices, and on larger ones the rows beyond the
+// shared table of k_contract_cta, window by window (at most kDenseWindows),
+// whose global table and global sort made a circuit graph's few hub rows the
+// last to finish (heavy rows of all levels of a 4M-vertex circuit graph 6.8
+// ms, now 2.7).
+constexpr i32 kDenseThreads = 1024;
+constexpr i32 kDenseIds = 53248;
+constexpr i32 kDenseWindows = 32;
+constexpr size_t kDenseSmem = (size_t)kDenseIds * 4 + kDenseIds / 8;
+constexpr i32 kCtaCap = 4096;   // k_contract_cta: longest row of its shared table
+
+__device__ __forceinline__ bool dense_row(i32 nc, i32 L) {
+  return nc <= kDenseIds || (L > kCtaCap && (i64)nc <= (i64)kDenseIds * kDenseWindows);
+}
+
+__global__ void __launch_bounds__(kDenseThreads, 1) k_contract_dense(
+    const i32* __restrict__ ncp, const i32* __restrict__ heavy, const i32* __restrict__ nheavy,
+    const i32* __restrict__ xadj, const i32* __restrict__ adjncy, const i32* __restrict__ adjwgt,
+    const i32* __restrict__ cmap, const i32* __restrict__ memtab, const i32* __restrict__ mcnt, i32 cap,
+    const i32* __restrict__ rowlen, const i32* __restrict__ ub, i32* __restrict__ sadj, i32* __restrict__ swgt,
+    i32* __restrict__ cnt) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  u32* acc = reinterpret_cast<u32*>(smem_raw);         // [kDenseIds]
+  u32* bits = acc + kDenseIds;                         // [kDenseIds / 32]
+  __shared__ i32 s_warp[kDenseThreads / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const i32 nc = *ncp, nh = *nheavy;
+  if (nh == 0) return;
+  for (i32 x = threadIdx.x; x < kDenseIds + kDenseIds / 32; x += kDenseThreads) acc[x] = 0;   // bits follow acc
+  __syncthreads();
+  for (i32 b = blockIdx.x; b < nh; b += gridDim.x) {
+    const i32 c = heavy[b];
+    if (!dense_row(nc, rowlen[c])) continue;   // block-uniform
+    const i32 nm = mcnt[c], o = ub[c];
+    i32 U = 0;
+    for (i32 w0 = 0; w0 < nc; w0 += kDenseIds) {
+      const u32 wn = (u32)(nc - w0 < kDenseIds ? nc - w0 : kDenseIds);
+      for (i32 j0 = 0; j0 < nm; j0 += 4) {   // four member rows together
+        i32 beg[4], end[4];
+#pragma unroll
+        for (i32 q = 0; q < 4; ++q) {
+          const i32 v = j0 + q < nm ? memtab[c * (i64)cap + j0 + q] : -1;
+          beg[q] = v >= 0 ? xadj[v] + (i32)threadIdx.x : 0;
+          end[q] = v >= 0 ? xadj[v + 1] : 0;
+        }
+        bool more = true;
+        while (more) {
+          i32 u[4], w[4];
+#pragma unroll
+          for (i32 q = 0; q < 4; ++q) {
+            u[q] = beg[q] < end[q] ? adjncy[beg[q]] : -1;
+            w[q] = beg[q] < end[q] ? adjwgt[beg[q]] : 0;
+          }
+#pragma unroll
+          for (i32 q = 0; q < 4; ++q) u[q] = u[q] >= 0 ? cmap[u[q]] : -1;
+          more = false;
+#pragma unroll
+          for (i32 q = 0; q < 4; ++q) {
+            const u32 id = (u32)(u[q] - w0);
+            if (u[q] >= 0 && u[q] != c && id < wn) {
+              atomicAdd(&acc[id], (u32)w[q]);
+              atomicOr(&bits[id >> 5], 1u << (id & 31));
+            }
+            beg[q] += kDenseThreads;
+            more |= beg[q] < end[q];
+          }
+        }
+      }
+      __syncthreads();
+      // the met ids in order: kDenseIds / 32 / kDenseThreads words a thread
+      constexpr i32 kW = (kDenseIds / 32 + kDenseThreads - 1) / kDenseThreads;
+      const i32 x0 = (i32)threadIdx.x * kW;
+      u32 word[kW];
+      i32 n = 0;
+#pragma unroll
+      for (i32 q = 0; q < kW; ++q) {
+        word[q] = x0 + q < kDenseIds / 32 ? bits[x0 + q] : 0u;
+        n += __popc(word[q]);
+      }
+      i32 inc = n;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const i32 y = __shfl_up_sync(kFull, inc, d);
+        if (lane >= d) inc += y;
+      }
+      if (lane == 31) s_warp[wid] = inc;
+      __syncthreads();
+      i32 before = 0, tot = 0;
+      for (i32 w = 0; w < kDenseThreads / 32; ++w) {
+        const i32 y = s_warp[w];
+        before += w < wid ? y : 0;
+        tot += y;
+      }
+      i32 at = o + U + before + inc - n;
+#pragma unroll
+      for (i32 q = 0; q < kW; ++q) {
+        if (word[q]) bits[x0 + q] = 0;
+        for (u32 m = word[q]; m; m &= m - 1) {
+          const i32 id = ((x0 + q) << 5) + __ffs(m) - 1;
+          sadj[at] = w0 + id;
+          swgt[at] = (i32)acc[id];
+          acc[id] = 0;
+          ++at;
+        }
+      }
+      U += tot;
+      __syncthreads();   // acc and bits are clear; s_warp is free
+    }
+    if (threadIdx.x == 0) cnt[c] = U;
+  }
+}
+
 // One CTA per heavy coarse row.  Table in dynamic shared memory when the row
 // fits (L <= cta_cap); longer rows take their table from the handle's arena
 // (bump allocation: keys and values of hsz words each, then hsz/2 sorted
@@ -935,7 +1109,7 @@ __global__ void __launch_bounds__(WARPS * 32) k_contract_warp(
 // needs and sets the overflow flag; the host grows the arena and runs the
 // contraction again.  Both kinds of row run in one launch.
 __global__ void __launch_bounds__(512) k_contract_cta(
-    const i32* __restrict__ heavy, const i32* __restrict__ nheavy, i32 cta_cap,
+    const i32* __restrict__ ncp, const i32* __restrict__ heavy, const i32* __restrict__ nheavy, i32 cta_cap,
     const i32* __restrict__ xadj, const i32* __restrict__ adjncy, const i32* __restrict__ adjwgt,
     const i32* __restrict__ cmap, const i32* __restrict__ memtab, const i32* __restrict__ mcnt, i32 cap,
     const i32* __restrict__ rowlen, const i32* __restrict__ ub, i32* __restrict__ sadj,
@@ -943,10 +1117,11 @@ __global__ void __launch_bounds__(512) k_contract_cta(
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ i32 s_count;
   __shared__ u64 s_off;
-  const i32 nh = *nheavy;
+  const i32 nc = *ncp, nh = *nheavy;
   for (i32 b = blockIdx.x; b < nh; b += gridDim.x) {
     const i32 c = heavy[b];
     const i32 L = rowlen[c];
+    if (dense_row(nc, L)) continue;   // k_contract_dense takes it (block-uniform)
     const bool global_table = L > cta_cap;   // block-uniform
     u32 hsz = 64;
     while (hsz < 2u * (u32)L) hsz <<= 1;
@@ -1013,13 +1188,18 @@ __global__ void __launch_bounds__(512) k_contract_cta(
   }
 }
 
-// One warp per 32 consecutive coarse rows: the lanes scan the rows' lengths
-// and copy the 32 rows' entries as one flat range, each lane finding its
-// entry's row by a binary search over the lanes' prefix sums.  A hub row of
-// thousands of entries is then copied by all 32 lanes, not by one thread.
+// One warp per R consecutive coarse rows (R <= 32): the lanes scan the rows'
+// lengths and copy the R rows' entries as one flat range, each lane finding
+// its entry's row by a binary search over the lanes' prefix sums.  R is small
+// on levels of long rows: a dense level has few rows, and 32 of 1000 entries
+// kept one warp for 32k (all levels of a 4M-vertex circuit graph: 4.4 ms, now
+// 0.9).  On levels of up to 100k vertices R = 8 (or 4) gives more warps a
+// shorter chain (2048 vertices: 7.6 us, now 5.3; on a million R = 8 is 2.6x
+// slower than 32).
 // Also the level's longest coarse row and heaviest coarse vertex (both
 // *maxdeg and *max_cvw start at zero).
-__global__ void k_copy_rows(const i32* __restrict__ ncp, const i32* __restrict__ ub, const i32* __restrict__ cnt,
+__global__ void k_copy_rows(const i32* __restrict__ ncp, i32 R, const i32* __restrict__ ub,
+                            const i32* __restrict__ cnt,
                             const i32* __restrict__ cx, const i32* __restrict__ sadj,
                             const i32* __restrict__ swgt, i32* __restrict__ cadj, i32* __restrict__ cwgt,
                             i32* __restrict__ maxdeg, const i32* __restrict__ cvw, i32* __restrict__ max_cvw) {
@@ -1028,10 +1208,10 @@ __global__ void k_copy_rows(const i32* __restrict__ ncp, const i32* __restrict__
   const i64 warp = ((i64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const i64 nwarps = ((i64)gridDim.x * blockDim.x) >> 5;
   i32 mx = 0, mw = 0;
-  for (i64 c0 = warp * 32; c0 < nc; c0 += nwarps * 32) {
+  for (i64 c0 = warp * R; c0 < nc; c0 += nwarps * R) {
     const i64 c = c0 + lane;
     i32 src = 0, dst = 0, len = 0;
-    if (c < nc) {
+    if (lane < R && c < nc) {
       src = ub[c];
       dst = cx[c];
       len = cnt[c];
@@ -1046,6 +1226,26 @@ __global__ void k_copy_rows(const i32* __restrict__ ncp, const i32* __restrict__
     }
     const i32 total = __shfl_sync(kFull, inc, 31);
     const i32 exc = inc - len;
+    if (R == 1) {   // one row: a straight copy, four entries a lane together
+      const i32 rs = __shfl_sync(kFull, src, 0), rd = __shfl_sync(kFull, dst, 0);
+      constexpr i32 kU = 4;
+      for (i32 e0 = lane; e0 < total; e0 += 32 * kU) {
+        i32 x[kU], y[kU];
+#pragma unroll
+        for (i32 q = 0; q < kU; ++q)
+          if (e0 + 32 * q < total) {
+            x[q] = sadj[rs + e0 + 32 * q];
+            y[q] = swgt[rs + e0 + 32 * q];
+          }
+#pragma unroll
+        for (i32 q = 0; q < kU; ++q)
+          if (e0 + 32 * q < total) {
+            cadj[rd + e0 + 32 * q] = x[q];
+            cwgt[rd + e0 + 32 * q] = y[q];
+          }
+      }
+      continue;
+    }
     for (i32 base = 0; base < total; base += 32) {   // warp-uniform: every lane takes every shuffle
       const i32 idx = base + lane;
       // the row r with exc_r <= idx < inc_r: the first lane whose inclusive sum exceeds idx
@@ -1100,7 +1300,8 @@ void run_contract(Handle& h, const DevGraph& g, const i32* cmap, const i32* d_nc
   i32* memtab = h.scratch.alloc_n<i32>((i64)nc_ub * cap + 1);
   i32* cnt = h.scratch.alloc_n<i32>(nu);
   i32* heavy = h.scratch.alloc_n<i32>(nu);
-  i32* misc = h.scratch.alloc_n<i32>(8);   // [0] heavy rows, [1] ub total
+  i32* mid = h.scratch.alloc_n<i32>(nu);
+  i32* misc = h.scratch.alloc_n<i32>(8);   // [0] heavy rows, [1] ub total, [2] rows listed by the short kernel
   i32* sadj = h.scratch.alloc_n<i32>(std::max<i64>(g.m, 1));
   i32* swgt = h.scratch.alloc_n<i32>(std::max<i64>(g.m, 1));
   ensure_arena(h, u64(4) << 20);   // 16 MB of long-row tables to start with
@@ -1113,37 +1314,69 @@ void run_contract(Handle& h, const DevGraph& g, const i32* cmap, const i32* d_nc
     launch(k_coarse_accum, nb, 256, 0, h.stream, n, g.xadj, g.vwgt, cmap, cap, cvwgt, rowlen, mcnt, memtab, h.arena);
   GKW_CHECK_LAUNCH();
   exclusive_scan_i32(h, rowlen, ub, nu, misc + 1);   // rows beyond n_c have length 0
-  const double avgL = nc_ub ? (double)g.m / nc_ub : 0.0;
+  // Expected coarse row: a group's members (about five; at most cap) times the
+  // mean degree.  Short rows take 16 lanes each (12M-vertex road graph, 7
+  // entries a row: 3.2 ms with a warp each, now 1.4 over all levels); else one
+  // warp per row with a table of 128 entries, 256 or 512.  A 27-point grid's
+  // rows have up to 156: with 128 nearly all went to one CTA each, 6.5 ms, now
+  // 0.73; above 400 expected the 512 table keeps more rows out of the heavy
+  // list, below it 256 lets four CTAs share an SM (2.9 -> 0.8 ms on the
+  // circuit graph's third level).
+  const double avg = n ? (double)g.m / n : 0.0;
+  const double expL = avg * std::min(cap, 6);
   const u32 gridw = std::max<u32>(1, std::min<u32>(ceil_div(std::max(nc_ub, 1), 8), (u32)h.sm_count * 32));
   u32* words = reinterpret_cast<u32*>(h.arena + 1);
-  if (avgL <= 48) {
-    constexpr int W = 128, WARPS = 8;
-    const size_t sm = sizeof(WarpTable<W>) * WARPS;
-    if (!h.capturing)
-      GKW_CUDA(cudaFuncSetAttribute(k_contract_warp<W, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    launch(k_contract_warp<W, WARPS>, gridw, WARPS * 32, sm, h.stream, d_nc, g.xadj, g.adjncy, g.adjwgt, cmap,
-           memtab, mcnt, cap, rowlen, ub, sadj, swgt, cnt, heavy, misc);
-  } else {
-    constexpr int W = 512, WARPS = 8;
-    const size_t sm = sizeof(WarpTable<W>) * WARPS;
-    if (!h.capturing)
-      GKW_CUDA(cudaFuncSetAttribute(k_contract_warp<W, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    launch(k_contract_warp<W, WARPS>, gridw, WARPS * 32, sm, h.stream, d_nc, g.xadj, g.adjncy, g.adjwgt, cmap,
-           memtab, mcnt, cap, rowlen, ub, sadj, swgt, cnt, heavy, misc);
+  const bool wide_ids = n >= (1 << 27);   // (id, lane) keys of 64 bits
+  const i32* rows = d_nc;
+  const i32* list = nullptr;
+  const bool shorts = expL <= 20 && cap <= kContractG;
+  if (shorts) {
+    auto go = [&](auto kern) {
+      launch(kern, std::max<u32>(1, std::min<u32>(ceil_div(std::max(nc_ub, 1), 16), (u32)h.sm_count * 32)), 256, 0,
+             h.stream, d_nc, g.xadj, g.adjncy, g.adjwgt, cmap, memtab, mcnt, cap, rowlen, ub, sadj, swgt, cnt, mid,
+             misc + 2);
+    };
+    if (wide_ids) go(k_contract_short<u64>);
+    else go(k_contract_short<u32>);
+    rows = misc + 2;
+    list = mid;
   }
+  auto warps = [&](auto w, auto k) {
+    constexpr int W = decltype(w)::value, WARPS = 8;
+    typedef decltype(k) K;
+    const size_t sm = sizeof(WarpTable<W>) * WARPS;
+    auto kern = k_contract_warp<W, WARPS, K>;
+    if (!h.capturing)
+      GKW_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    launch(kern, gridw, WARPS * 32, sm, h.stream, rows, list, g.xadj, g.adjncy, g.adjwgt, cmap, memtab, mcnt, cap,
+           rowlen, ub, sadj, swgt, cnt, heavy, misc);
+  };
+  if (wide_ids) warps(std::integral_constant<int, 128>(), u64());
+  else if (expL <= 100) warps(std::integral_constant<int, 128>(), u32());   // (W below)
+  else if (expL <= 400) warps(std::integral_constant<int, 256>(), u32());
+  else warps(std::integral_constant<int, 512>(), u32());
   GKW_CHECK_LAUNCH();
-  // heavy rows: a shared-memory table up to kCtaCap entries, the arena beyond
-  // (2*kCtaCap table slots, a power of two, + kCtaCap sorted outputs: 96 KB)
-  constexpr i32 kCtaCap = 4096;
-  const size_t csm = (size_t)kCtaCap * 2 * 4 * 2 + (size_t)kCtaCap * 8;
-  if (!h.capturing)
-    GKW_CUDA(cudaFuncSetAttribute(k_contract_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
-  launch(k_contract_cta, (u32)h.sm_count * 2, 512, csm, h.stream, heavy, misc, kCtaCap, g.xadj, g.adjncy,
-         g.adjwgt, cmap, memtab, mcnt, cap, rowlen, ub, sadj, swgt, cnt, h.arena, words, h.arena_words);
-  GKW_CHECK_LAUNCH();
+  // heavy rows: only where a row can outgrow the warp tables.  A shared-memory
+  // table up to kCtaCap entries, the arena beyond (2*kCtaCap table slots, a
+  // power of two, + kCtaCap sorted outputs: 96 KB)
+  const i32 W = wide_ids || expL <= 100 ? 128 : expL <= 400 ? 256 : 512;
+  if (g.maxdeg < 0 || g.maxdeg * (i64)cap > W || cap > 32) {
+    const size_t csm = (size_t)kCtaCap * 2 * 4 * 2 + (size_t)kCtaCap * 8;
+    if (!h.capturing) {
+      GKW_CUDA(cudaFuncSetAttribute(k_contract_dense, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem));
+      GKW_CUDA(cudaFuncSetAttribute(k_contract_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
+    }
+    launch(k_contract_dense, (u32)h.sm_count, kDenseThreads, kDenseSmem, h.stream, d_nc, heavy, misc, g.xadj,
+           g.adjncy, g.adjwgt, cmap, memtab, mcnt, cap, rowlen, ub, sadj, swgt, cnt);
+    if (nc_ub > kDenseIds)
+      launch(k_contract_cta, (u32)h.sm_count * 2, 512, csm, h.stream, d_nc, heavy, misc, kCtaCap, g.xadj, g.adjncy,
+             g.adjwgt, cmap, memtab, mcnt, cap, rowlen, ub, sadj, swgt, cnt, h.arena, words, h.arena_words);
+    GKW_CHECK_LAUNCH();
+  }
   exclusive_scan_i32(h, cnt, cxadj, nu, d_mc);   // cxadj[n_c] = m_c (rows beyond n_c are empty)
+  const i32 R = expL > 200 ? 1 : nc_ub > 100000 ? 32 : expL <= 48 ? 8 : 4;
   if (nc_ub > 0)
-    launch(k_copy_rows, ceil_div(nc_ub, 256), 256, 0, h.stream, d_nc, ub, cnt, cxadj, sadj, swgt, cadjncy,
+    launch(k_copy_rows, std::min<u32>(ceil_div((u64)nc_ub, 8 * (u64)R), (u32)h.sm_count * 32), 256, 0, h.stream, d_nc, R, ub, cnt, cxadj, sadj, swgt, cadjncy,
            cadjwgt, &h.coop->maxdeg, (const i32*)cvwgt, &h.coop->max_cvw);
   GKW_CHECK_LAUNCH();
   h.scratch.release(mk);
