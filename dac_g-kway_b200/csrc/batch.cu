@@ -249,14 +249,14 @@ bool partition_batch_union(Handle& hh, const DevGraph& hg, i32 G, const i32* gra
   i32* a = hh.hier.alloc_n<i32>(std::max<i64>(m, 1));
   i32* w = hh.hier.alloc_n<i32>(std::max<i64>(m, 1));
   i32* vw = hh.hier.alloc_n<i32>(std::max<i64>(n, 1));
-  GKW_CUDA(cudaMemcpyAsync(x, hg.xadj, sizeof(i32) * (n + 1), cudaMemcpyHostToDevice, hh.stream));
+  copy_to_device(hh, x, hg.xadj, sizeof(i32) * (n + 1));
   if (m) {
-    GKW_CUDA(cudaMemcpyAsync(a, hg.adjncy, sizeof(i32) * m, cudaMemcpyHostToDevice, hh.stream));
-    if (hg.adjwgt) GKW_CUDA(cudaMemcpyAsync(w, hg.adjwgt, sizeof(i32) * m, cudaMemcpyHostToDevice, hh.stream));
+    copy_to_device(hh, a, hg.adjncy, sizeof(i32) * m);
+    if (hg.adjwgt) copy_to_device(hh, w, hg.adjwgt, sizeof(i32) * m);
     else launch(k_fill_one, ceil_div(m, 256), 256, 0, hh.stream, w, m);
   }
   if (n) {
-    if (hg.vwgt) GKW_CUDA(cudaMemcpyAsync(vw, hg.vwgt, sizeof(i32) * n, cudaMemcpyHostToDevice, hh.stream));
+    if (hg.vwgt) copy_to_device(hh, vw, hg.vwgt, sizeof(i32) * n);
     else launch(k_fill_one, ceil_div(n, 256), 256, 0, hh.stream, vw, n);
   }
   GKW_CHECK_LAUNCH();
@@ -584,7 +584,7 @@ bool partition_batch_union(Handle& hh, const DevGraph& hg, i32 G, const i32* gra
   GKW_CUDA(cudaMemsetAsync(cut, 0, sizeof(u64) * G, hh.stream));
   launch(k_graph_cut, ceil_div(n, 256), 256, 0, hh.stream, (i32)n, x, a, w, lv[0].gid, part, cut);
   GKW_CHECK_LAUNCH();
-  GKW_CUDA(cudaMemcpyAsync(part_out, loc, sizeof(i32) * n, cudaMemcpyDeviceToHost, hh.stream));
+  copy_to_host(hh, part_out, loc, sizeof(i32) * (size_t)n);
   const std::vector<unsigned long long> hc = to_host(hh, cut, G);
   for (i32 i = 0; i < G; ++i) {
     if (cuts_out) cuts_out[i] = (i64)hc[i];

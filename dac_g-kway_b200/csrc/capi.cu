@@ -164,6 +164,7 @@ gkw_status gkw_destroy(gkw_handle* h) {
     cudaStreamSynchronize(h->h.stream);
     if (h->h.own_stream) cudaStreamDestroy(h->h.stream);
     cudaFreeHost(h->h.h_pinned);
+    free_stage(h->h);
     if (h->h.scan) cudaFree(h->h.scan);
     if (h->h.coop) cudaFree(h->h.coop);
     if (h->h.arena) cudaFree(h->h.arena);

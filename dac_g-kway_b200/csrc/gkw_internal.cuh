@@ -209,6 +209,14 @@ struct Handle {
   bool narrow = false;
   cudaEvent_t coop_ev = nullptr;   // this handle's last wide cooperative launch
   gkw_tuning tuning{{4, 8, 16, 32}, 512, 32, 0, 256};   // launch shapes (gkw_autotune)
+  // Pinned staging for pageable host memory and files (copy_to_device and
+  // stage_buffer, common.cu): made on first use, at most kStageBytes, freed
+  // with the handle
+  char* stage = nullptr;
+  size_t stage_cap = 0;
+  bool stage_raw = false;   // handed out by stage_buffer: its copies have no slot events
+  static constexpr int kStageSlots = 16;
+  cudaEvent_t stage_ev[kStageSlots] = {};   // last copy out of (or into) each slot
   // while the autotuner collects: per average-degree bucket, the summed time
   // of each match lane count (4, 8, 16, 32) over the levels met
   bool tune_collect = false;
@@ -216,6 +224,20 @@ struct Handle {
   Handle() : hier(size_t(256) << 20), scratch(size_t(256) << 20) {}
 };
 void ensure_timer_events(Handle& h);
+
+// ---- host memory (common.cu) ----
+constexpr size_t kStageChunk = size_t(2) << 20;
+constexpr size_t kStageBytes = kStageChunk * Handle::kStageSlots;   // 32 MB
+// A pinned buffer of at least `bytes` that the handle keeps, or null above
+// kStageBytes.  Valid until the next staged copy or stage_buffer call.
+char* stage_buffer(Handle& h, size_t bytes);
+void free_stage(Handle& h);
+// Host-to-device copy on the handle's stream.  Large pageable sources go
+// through the pinned slots, filled by several threads; the source is free
+// when the call returns, the copy itself may still be queued.
+void copy_to_device(Handle& h, void* dst, const void* src, size_t bytes);
+// Device-to-host copy of queued results; complete when the call returns.
+void copy_to_host(Handle& h, void* dst, const void* src, size_t bytes);
 
 // ---- kernels with grid barriers (common.cu) ----
 // Largest thread-block cluster the kernel can be launched as with this block

@@ -351,8 +351,19 @@ namespace {
 
 struct PinnedBuf {
   char* p = nullptr;
+  bool own = false;
+  void get(Handle& h, size_t bytes) {
+    p = stage_buffer(h, bytes);
+    if (p) return;
+    if (cudaHostAlloc((void**)&p, bytes, cudaHostAllocDefault) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+      throw Error{GKW_E_NOMEM, "cannot allocate pinned memory for the graph file"};
+    }
+    own = true;
+  }
   ~PinnedBuf() {
-    if (p) cudaFreeHost(p);
+    if (own) cudaFreeHost(p);
   }
 };
 
@@ -377,10 +388,11 @@ void read_metis_device(Handle& h, const char* path, bool quirks, DeviceCsr& out)
   fseek(f, 0, SEEK_SET);
   PinnedBuf hb;
   const size_t size = sz > 0 ? (size_t)sz : 0;
-  if (cudaHostAlloc((void**)&hb.p, std::max<size_t>(size, 1), cudaHostAllocDefault) != cudaSuccess) {
+  try {   // the handle's staging buffer, or one of its own for a large file
+    hb.get(h, std::max<size_t>(size, 1));
+  } catch (...) {
     fclose(f);
-    cudaGetLastError();
-    throw Error{GKW_E_NOMEM, "cannot allocate pinned memory for the graph file"};
+    throw;
   }
   const size_t got = size ? fread(hb.p, 1, size, f) : 0;
   fclose(f);
@@ -501,7 +513,7 @@ void write_partition_device(Handle& h, const char* path, i32 n, const i32* d_par
   if (n > 0) launch(k_id_text, ceil_div(n, 256), 256, 0, h.stream, n, d_part, (const i32*)off, text);
   GKW_CHECK_LAUNCH();
   PinnedBuf hb;
-  GKW_CUDA(cudaHostAlloc((void**)&hb.p, std::max<size_t>(bytes, 1), cudaHostAllocDefault));
+  hb.get(h, std::max<size_t>(bytes, 1));
   if (bytes) GKW_CUDA(cudaMemcpyAsync(hb.p, text, (size_t)bytes, cudaMemcpyDeviceToHost, h.stream));
   GKW_CUDA(cudaStreamSynchronize(h.stream));
   h.scratch.release(mk);

@@ -572,23 +572,23 @@ DevGraph upload_host_graph(Handle& hh, const DevGraph& hg, i64 vbase) {
   i32* a = hh.hier.alloc_n<i32>(std::max<i64>(m, 1));
   i32* w = hh.hier.alloc_n<i32>(std::max<i64>(m, 1));
   i32* vw = hh.hier.alloc_n<i32>(std::max<i64>(n, 1));
-  GKW_CUDA(cudaMemcpyAsync(x, hg.xadj, sizeof(i32) * (n + 1), cudaMemcpyHostToDevice, hh.stream));
+  copy_to_device(hh, x, hg.xadj, sizeof(i32) * (n + 1));
   const i32 ebase = hg.xadj[0];
   if (ebase != 0) {
     launch(k_sub_i32, ceil_div(n + 1, 256), 256, 0, hh.stream, x, n + 1, ebase);
     GKW_CHECK_LAUNCH();
   }
   if (m) {
-    GKW_CUDA(cudaMemcpyAsync(a, hg.adjncy, sizeof(i32) * m, cudaMemcpyHostToDevice, hh.stream));
+    copy_to_device(hh, a, hg.adjncy, sizeof(i32) * m);
     if (vbase != 0) {
       launch(k_sub_i32, ceil_div(m, 256), 256, 0, hh.stream, a, m, (i32)vbase);
       GKW_CHECK_LAUNCH();
     }
-    if (hg.adjwgt) GKW_CUDA(cudaMemcpyAsync(w, hg.adjwgt, sizeof(i32) * m, cudaMemcpyHostToDevice, hh.stream));
+    if (hg.adjwgt) copy_to_device(hh, w, hg.adjwgt, sizeof(i32) * m);
     else launch(k_fill_i32, ceil_div(m, 256), 256, 0, hh.stream, w, m, 1);
   }
   if (n) {
-    if (hg.vwgt) GKW_CUDA(cudaMemcpyAsync(vw, hg.vwgt, sizeof(i32) * n, cudaMemcpyHostToDevice, hh.stream));
+    if (hg.vwgt) copy_to_device(hh, vw, hg.vwgt, sizeof(i32) * n);
     else launch(k_fill_i32, ceil_div(n, 256), 256, 0, hh.stream, vw, n, 1);
   }
   GKW_CHECK_LAUNCH();
@@ -614,8 +614,7 @@ void partition_host(Handle& hh, const DevGraph& hg, i64 vbase, i32 k, const gkw_
   const DevGraph g = upload_host_graph(hh, hg, vbase);
   i32* part = hh.hier.alloc_n<i32>(std::max<i64>(hg.n, 1));
   partition_impl(hh, g, k, o, part, cut_out, stats);
-  if (hg.n) GKW_CUDA(cudaMemcpyAsync(part_out, part, sizeof(i32) * hg.n, cudaMemcpyDeviceToHost, hh.stream));
-  GKW_CUDA(cudaStreamSynchronize(hh.stream));
+  copy_to_host(hh, part_out, part, sizeof(i32) * (size_t)hg.n);
 }
 
 // Several k over one hierarchy, host arrays in and out (nk rows of n ids).
@@ -627,9 +626,7 @@ void partition_multi_host(Handle& hh, const DevGraph& hg, i32 nk, const i32* ks,
   const DevGraph g = upload_host_graph(hh, hg, 0);
   i32* parts = hh.hier.alloc_n<i32>(std::max<i64>((i64)hg.n * std::max(nk, 1), 1));
   partition_multi_impl(hh, g, nk, ks, o, parts, cuts_out);
-  if (hg.n && nk)
-    GKW_CUDA(cudaMemcpyAsync(parts_out, parts, sizeof(i32) * (size_t)hg.n * nk, cudaMemcpyDeviceToHost, hh.stream));
-  GKW_CUDA(cudaStreamSynchronize(hh.stream));
+  copy_to_host(hh, parts_out, parts, sizeof(i32) * (size_t)hg.n * nk);
 }
 
 }  // namespace gkw
