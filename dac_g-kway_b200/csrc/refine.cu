@@ -1880,8 +1880,7 @@ __device__ __forceinline__ u64 block_reduce_u64(u64 x, u64* s_tmp) {
   return r;
 }
 
-constexpr i32 kRiskEvents = 1024;   // event limit of the at-risk balance check
-constexpr i32 kRiskParts = 1024;    // part limit of that check (k)
+constexpr i32 kRiskParts = 1024;    // part limit of the at-risk balance check (k)
 constexpr i32 kRiskCands = 1024;    // candidate limit of that check
 
 // The balance check of a round whose candidates are all kept (cnt <= cap),
@@ -1893,185 +1892,194 @@ constexpr i32 kRiskCands = 1024;    // candidate limit of that check
 //    moves.  A flagged part's change at the last index is its net change
 //    over all candidates (pnet).
 //  * Otherwise each move into or out of a flagged part is an event (part,
-//    key, +-w), the events are grouped by part (a counting sort), and a
-//    part's D after one of its events is the sum of its events with keys up
-//    to that key, which holds until the part's next event; an event with
-//    D > 0 and (float)(pw + D) > MAXW marks the key range [key, next key of
-//    the part) -- the index ranges the reference's table marks
-//    (uncoarsen.hpp:239-288), in key order.  Every candidate key is tested
-//    against the marked ranges, and the moves with key <= K* apply, K* = the
-//    largest unmarked key, or the smallest key if all are marked (prefix 0
-//    always counts as balanced, :481-488).
-// All global loads come first and at once, from two halves of the CTA: warps
-// 0-7 fetch the candidate list entries (key, source, destination, weight,
-// written beside each other by the candidates phase), warps 8-15 every
-// part's flag, net change and weight.  Everything after one block barrier is
-// shared memory.  Returns false (block-uniform) when the last index is not
-// balanced and k > kRiskParts, cnt > kRiskCands or the events exceed
-// kRiskEvents; the caller then runs the check over all parts.
-__device__ bool refine_check_risk(const LevelArgs& a, i32 cnt, u64* s, i32* greedy, u64* keep, u64* s_tmp,
-                                  u32* s_warp, u64* kstar, i32* napplied) {
-  __shared__ i32 s_ne, s_nbad, s_lastbad;
-  constexpr i32 kHalf = kLevelThreads / 2;
-  constexpr i32 kPerThread = kRiskCands / kHalf;   // candidates per loading thread
-  static_assert(kRiskCands % kHalf == 0, "candidates split evenly over the loading threads");
-  u64* ev_key = s + kMaxMoveCap;      // [kRiskEvents] events as found
-  u64* gk = ev_key + kRiskEvents;     // [kRiskEvents] grouped by part
-  u64* bad_lo = keep;                 // [kRiskEvents] marked key ranges [lo, hi)
-  u64* bad_hi = keep + kRiskEvents;   // [kRiskEvents]
-  i32* ev_b = greedy;                 // [kRiskEvents] part of each event
-  i32* ev_d = ev_b + kRiskEvents;     // [kRiskEvents] weight change
-  i32* gb = ev_d + kRiskEvents;       // grouped: part
-  i32* gd = gb + kRiskEvents;         // grouped: weight change
-  i32* bcnt = gd + kRiskEvents;       // [kRiskParts] events per part
-  i32* boff = bcnt + kRiskParts;      // [kRiskParts] first grouped slot
-  i32* bfill = boff + kRiskParts;     // [kRiskParts]
-  i32* rpw = bfill + kRiskParts;      // [kRiskParts] part weight before the round
-  i32* rflag = rpw + kRiskParts;      // [kRiskParts] part flagged in risk
-  static_assert(4 * kRiskEvents + 5 * kRiskParts <= kGreedyWords, "check arrays fit the greedy region");
-  static_assert(kMaxMoveCap + 2 * kRiskEvents <= kSortMax, "event keys fit the sort buffer");
-  static_assert(kRiskCands <= kMaxMoveCap, "candidate keys fit the sort buffer");
+//    key, +-w), the events are grouped by part, and a part's D after one of
+//    its events is the sum of its events with keys up to that key, which
+//    holds until the part's next event; an event with D > 0 and
+//    (float)(pw + D) > MAXW marks the key range [key, next key of the part)
+//    -- the index ranges the reference's table marks (uncoarsen.hpp:239-288),
+//    in key order.  Every candidate key is tested against the marked ranges,
+//    and the moves with key <= K* apply, K* = the largest unmarked key, or the
+//    smallest key if all are marked (prefix 0 always counts as balanced,
+//    :481-488).
+// Every CTA that owns a move waits for this chain, so it is kept short: a
+// thread's candidates and parts are loaded beside the round's check flag (by
+// the caller), the count of a part's events hands out their places in it (one
+// atomic each, no event list), the range tests run without early exits, and
+// the two maxima are warp reductions joined once: 2^20-vertex mesh, k = 64
+// (160 candidates, 72 events, 14 ranges a round on average): MEASURE_CHECK.
+// Returns false (block-uniform) when the last index is not balanced and k >
+// kRiskParts or cnt > kRiskCands; the caller then runs the check over all
+// parts.  *napplied is set on block 0 only.
+constexpr i32 kRiskPer = kRiskCands / kLevelThreads;   // candidates, and parts, of a thread
+static_assert(kRiskParts == kRiskCands && kRiskCands % kLevelThreads == 0, "an equal share per thread");
+struct RiskLoads {
+  u64 key[kRiskPer], inf[kRiskPer];
+  i32 w[kRiskPer], net[kRiskPer];
+  u32 risk[kRiskPer], pw[kRiskPer];
+};
+__device__ __forceinline__ void risk_loads(const LevelArgs& a, i32 cnt, RiskLoads& L) {
+#pragma unroll
+  for (i32 q = 0; q < kRiskPer; ++q) {
+    const i32 i = (i32)threadIdx.x + q * kLevelThreads;
+    L.key[q] = L.inf[q] = 0;
+    L.w[q] = L.net[q] = 0;
+    L.risk[q] = L.pw[q] = 0;
+    if (i < cnt) {
+      L.key[q] = ldc(a.cands + i);
+      L.inf[q] = ldc(a.cinfo + i);
+      L.w[q] = ldc(a.cw + i);
+    }
+    if (i < a.k) {
+      L.risk[q] = ldc(a.risk + i);
+      L.net[q] = ldc(a.pnet + i);
+      L.pw[q] = ldc(a.pw + i);
+    }
+  }
+}
+
+__device__ bool refine_check_risk(const LevelArgs& a, i32 cnt, const RiskLoads& L, u64* s, i32* greedy, u64* keep,
+                                  u64* s_tmp, u32* s_warp, u64* kstar, i32* napplied) {
+  __shared__ i32 s_nbad;
+  u64* ek = s;                                             // [2 * kRiskCands] events grouped by part: key
+  i32* ew = reinterpret_cast<i32*>(s + 2 * kRiskCands);    // [2 * kRiskCands] weight change
+  ulonglong2* bad = reinterpret_cast<ulonglong2*>(greedy); // [2 * kRiskCands] marked key ranges [x, y)
+  i32* rflag = reinterpret_cast<i32*>(keep);               // [kRiskParts] part flagged in risk
+  i32* rpw = rflag + kRiskParts;                           // [kRiskParts] part weight before the round
+  i32* bcnt = rpw + kRiskParts;                            // [kRiskParts] events of the part
+  i32* boff = bcnt + kRiskParts;                           // [kRiskParts] first of them
+  static_assert(2 * kRiskCands * 12 <= kSortMax * 8, "events fit the sort buffer");
+  static_assert(2 * kRiskCands * 16 <= kGreedyWords * 4, "ranges fit the greedy region");
+  static_assert(4 * kRiskParts * 4 <= kMaxMoveCap * 8, "part tables fit the kept moves' buffer");
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const i32 k = a.k;
   const bool small = k <= kRiskParts && cnt <= kRiskCands;   // block-uniform
-  if (threadIdx.x == 0) {
-    s_ne = 0;
-    s_nbad = 0;
-    s_lastbad = 0;
-  }
-  if (small)
-    for (i32 b = threadIdx.x; b < k; b += blockDim.x) {
-      bcnt[b] = 0;
-      bfill[b] = 0;
-    }
-  __syncthreads();
-  u64 key[kPerThread];
-  i32 src[kPerThread], dst[kPerThread], w[kPerThread];
-  if (threadIdx.x < kHalf) {
-    if (small) {
+  bool lastbad = false;
+  auto over = [&](u32 flag, i32 net, u32 pw) { return flag && net > 0 && __uint2float_rn((u32)net + pw) > a.maxw; };
 #pragma unroll
-      for (i32 q = 0; q < kPerThread; ++q) {
-        const i32 i = threadIdx.x + q * kHalf;
-        key[q] = ~0ull;
-        src[q] = dst[q] = w[q] = 0;
-        if (i < cnt) {
-          key[q] = ldc(a.cands + i);
-          const u64 inf = ldc(a.cinfo + i);
-          w[q] = ldc(a.cw + i);
-          src[q] = (i32)(u32)(inf >> 32);
-          dst[q] = (i32)(u32)inf;
-        }
-      }
-    }
-  } else {
-    bool bad = false;
-    for (i32 p = threadIdx.x - kHalf; p < k; p += kHalf) {
-      const u32 f = ldc(a.risk + p);
-      const i32 d = ldc(a.pnet + p);
-      const u32 pw = ldc(a.pw + p);
+  for (i32 q = 0; q < kRiskPer; ++q) {
+    const i32 p = (i32)threadIdx.x + q * kLevelThreads;
+    if (p < k) {
+      lastbad |= over(L.risk[q], L.net[q], L.pw[q]);
       if (small) {
-        rflag[p] = (i32)f;
-        rpw[p] = (i32)pw;
+        rflag[p] = (i32)L.risk[q];
+        rpw[p] = (i32)L.pw[q];
+        bcnt[p] = 0;
       }
-      if (f && d > 0 && __uint2float_rn((u32)d + pw) > a.maxw) bad = true;
     }
-    if (bad) s_lastbad = 1;
   }
-  __syncthreads();
-  if (!s_lastbad) {   // block-uniform: the last index is balanced, every candidate moves
+  for (i32 p = (i32)threadIdx.x + kRiskParts; p < k; p += kLevelThreads)
+    lastbad |= over(ldc(a.risk + p), ldc(a.pnet + p), ldc(a.pw + p));
+  if (threadIdx.x == 0) s_nbad = 0;
+  if (!__syncthreads_or((int)lastbad)) {   // the last index is balanced, every candidate moves
     *kstar = ~0ull;
     *napplied = cnt;
     return true;
   }
   if (!small) return false;
-  u64 kmin = ~0ull;
-  if (threadIdx.x < kHalf) {
+  // events: the part's count is the event's place in its group
+  i32 ps[kRiskPer], pd[kRiskPer];
 #pragma unroll
-    for (i32 q = 0; q < kPerThread; ++q) {
-      const i32 i = threadIdx.x + q * kHalf;
-      if (i >= cnt) continue;
-      s[i] = key[q];
-      kmin = key[q] < kmin ? key[q] : kmin;
-      if (rflag[src[q]]) {
-        const i32 e = atomicAdd(&s_ne, 1);
-        if (e < kRiskEvents) {
-          ev_key[e] = key[q];
-          ev_b[e] = src[q];
-          ev_d[e] = -w[q];
-          atomicAdd(&bcnt[src[q]], 1);
-        }
-      }
-      if (rflag[dst[q]]) {
-        const i32 e = atomicAdd(&s_ne, 1);
-        if (e < kRiskEvents) {
-          ev_key[e] = key[q];
-          ev_b[e] = dst[q];
-          ev_d[e] = w[q];
-          atomicAdd(&bcnt[dst[q]], 1);
-        }
-      }
+  for (i32 q = 0; q < kRiskPer; ++q) {
+    const i32 i = (i32)threadIdx.x + q * kLevelThreads;
+    ps[q] = pd[q] = -1;
+    if (i < cnt) {
+      const i32 sp = (i32)(u32)(L.inf[q] >> 32), dp = (i32)(u32)L.inf[q];
+      if (rflag[sp]) ps[q] = atomicAdd(&bcnt[sp], 1);
+      if (rflag[dp]) pd[q] = atomicAdd(&bcnt[dp], 1);
     }
   }
   __syncthreads();
-  trace_mark(a, 29);
-  const i32 ne = s_ne;
-  if (ne > kRiskEvents) return false;   // block-uniform
-  {   // first grouped slot of each part: exclusive scan, two parts per thread
-    const i32 b0 = 2 * threadIdx.x;
-    const u32 c0 = b0 < k ? (u32)bcnt[b0] : 0u, c1 = b0 + 1 < k ? (u32)bcnt[b0 + 1] : 0u;
-    u32 tot;
-    const u32 ex = block_exscan_u32(c0 + c1, s_warp, tot);
-    if (b0 < k) boff[b0] = (i32)ex;
-    if (b0 + 1 < k) boff[b0 + 1] = (i32)(ex + c0);
+  {   // first event of each part: a scan over kRiskPer parts a thread
+    const i32 b0 = kRiskPer * (i32)threadIdx.x;
+    i32 c[kRiskPer], loc = 0;
+#pragma unroll
+    for (i32 q = 0; q < kRiskPer; ++q) {
+      c[q] = b0 + q < k ? bcnt[b0 + q] : 0;
+      loc += c[q];
+    }
+    i32 inc = loc;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const i32 y = __shfl_up_sync(kFullMask, inc, o);
+      if (lane >= o) inc += y;
+    }
+    if (lane == 31) s_warp[wid] = (u32)inc;
+    __syncthreads();
+    i32 at = inc - loc;
+    for (i32 w = 0; w < wid; ++w) at += (i32)s_warp[w];
+#pragma unroll
+    for (i32 q = 0; q < kRiskPer; ++q) {
+      if (b0 + q < k) boff[b0 + q] = at;
+      at += c[q];
+    }
   }
   __syncthreads();
-  for (i32 e = threadIdx.x; e < ne; e += blockDim.x) {
-    const i32 b = ev_b[e];
-    const i32 at = boff[b] + atomicAdd(&bfill[b], 1);
-    gk[at] = ev_key[e];
-    gd[at] = ev_d[e];
-    gb[at] = b;
+#pragma unroll
+  for (i32 q = 0; q < kRiskPer; ++q) {
+    const i32 sp = (i32)(u32)(L.inf[q] >> 32), dp = (i32)(u32)L.inf[q];
+    if (ps[q] >= 0) {
+      ek[boff[sp] + ps[q]] = L.key[q];
+      ew[boff[sp] + ps[q]] = -L.w[q];
+    }
+    if (pd[q] >= 0) {
+      ek[boff[dp] + pd[q]] = L.key[q];
+      ew[boff[dp] + pd[q]] = L.w[q];
+    }
   }
   __syncthreads();
-  // marked key ranges
-  for (i32 j = threadIdx.x; j < ne; j += blockDim.x) {
-    const i32 b = gb[j];
-    const u64 kj = gk[j];
+  // marked key ranges, each move's event at its destination, then its source
+#pragma unroll
+  for (i32 q = 0; q < 2 * kRiskPer; ++q) {
+    const i32 b = (i32)(u32)((q & 1) ? L.inf[q >> 1] >> 32 : L.inf[q >> 1]);
+    if (((q & 1) ? ps[q >> 1] : pd[q >> 1]) < 0) continue;
+    const u64 kj = L.key[q >> 1];
     i32 D = 0;
     u64 knext = ~0ull;
-    for (i32 f = boff[b], fe = boff[b] + bcnt[b]; f < fe; ++f) {
-      const u64 kf = gk[f];
-      if (kf <= kj) D += gd[f];
-      else knext = kf < knext ? kf : knext;
+    const i32 f0 = boff[b], fe = f0 + bcnt[b];
+    for (i32 f = f0; f < fe; ++f) {
+      const u64 kf = ek[f];
+      const i32 wf = ew[f];
+      D += kf <= kj ? wf : 0;
+      knext = kf > kj && kf < knext ? kf : knext;
     }
-    if (D > 0 && __uint2float_rn((u32)D + (u32)rpw[b]) > a.maxw) {
-      const i32 at = atomicAdd(&s_nbad, 1);
-      bad_lo[at] = kj;
-      bad_hi[at] = knext;
-    }
+    if (D > 0 && __uint2float_rn((u32)D + (u32)rpw[b]) > a.maxw) bad[atomicAdd(&s_nbad, 1)] = make_ulonglong2(kj, knext);
   }
-  kmin = block_reduce_u64<false>(kmin, s_tmp);   // (its barriers publish the ranges)
-  trace_mark(a, 30);
-  const i32 nbad = s_nbad;
+  __syncthreads();
   // the largest candidate key in no marked range
-  u64 best = 0;
-  bool any = false;
-  for (i32 i = threadIdx.x; i < cnt; i += blockDim.x) {
-    const u64 kk = s[i];
-    bool marked = false;
-    for (i32 r = 0; r < nbad && !marked; ++r) marked = bad_lo[r] <= kk && kk < bad_hi[r];
-    if (!marked) {
-      best = kk > best ? kk : best;
-      any = true;
-    }
+  const i32 nbad = s_nbad;
+  bool marked[kRiskPer];
+#pragma unroll
+  for (i32 q = 0; q < kRiskPer; ++q) marked[q] = (i32)threadIdx.x + q * kLevelThreads >= cnt;
+#pragma unroll 4
+  for (i32 r = 0; r < nbad; ++r) {
+    const ulonglong2 x = bad[r];
+#pragma unroll
+    for (i32 q = 0; q < kRiskPer; ++q) marked[q] |= x.x <= L.key[q] && L.key[q] < x.y;
   }
-  const u64 top = block_reduce_u64<true>(any ? best + 1 : 0, s_tmp);   // +1: 0 means none
-  const u64 K = top ? top - 1 : kmin;
-  u32 c = 0;
-  for (i32 i = threadIdx.x; i < cnt; i += blockDim.x) c += s[i] <= K;
-  u32 tot;
-  (void)block_exscan_u32(c, s_warp, tot);
+  u64 best = 0;   // key + 1: 0 means none
+#pragma unroll
+  for (i32 q = 0; q < kRiskPer; ++q)
+    if (!marked[q] && L.key[q] >= best) best = L.key[q] + 1;
+  best = warp_max_key(best);
+  if (lane == 0) s_tmp[wid] = best;
+  __syncthreads();
+  u64 K = warp_max_key(lane < kLevelThreads / 32 ? s_tmp[lane] : 0ull);
+  if (K == 0) {   // block-uniform: every index is marked, the first move applies
+    u64 low = ~0ull;
+#pragma unroll
+    for (i32 q = 0; q < kRiskPer; ++q)
+      if ((i32)threadIdx.x + q * kLevelThreads < cnt) low = L.key[q] < low ? L.key[q] : low;
+    K = block_reduce_u64<false>(low, s_tmp) + 1;
+  }
+  K -= 1;
   *kstar = K;
-  *napplied = (i32)tot;
+  if (blockIdx.x == 0) {
+    i32 c = 0;
+#pragma unroll
+    for (i32 q = 0; q < kRiskPer; ++q)
+      c += __syncthreads_count((i32)threadIdx.x + q * kLevelThreads < cnt && L.key[q] <= K);
+    *napplied = c;
+  }
   return true;
 }
 
@@ -2104,6 +2112,8 @@ __device__ u32 ph_refine_apply(const LevelArgs& a, u64* s, i32* greedy, u64* kee
   // the warp's first candidate, loaded beside the check flag (used when every
   // candidate applies)
   const u64 key0 = warp < cnt ? ldc(a.cands + warp) : 0ull;
+  RiskLoads rl;   // the check's data, loaded beside its flag
+  risk_loads(a, cnt, rl);
   const bool check = ldc(&st->needcheck) != 0;
   __shared__ unsigned long long s_gsum;
   if (threadIdx.x == 0) {
@@ -2116,7 +2126,7 @@ __device__ u32 ph_refine_apply(const LevelArgs& a, u64* s, i32* greedy, u64* kee
   i32 pos = B - 1;     // sorted: moves 0..pos of keep apply
   if (check) {
     bool done = false;
-    if (cnt <= a.move_cap) done = refine_check_risk(a, cnt, s, greedy, keep, s_tmp, s_warp, &kstar, &napplied);
+    if (cnt <= a.move_cap) done = refine_check_risk(a, cnt, rl, s, greedy, keep, s_tmp, s_warp, &kstar, &napplied);
     trace_mark(a, 25);
     if (!done && a.k <= kRankParts && rank_select(a.cands, cnt, B, 0, a.n)) {
       trace_mark(a, 28);
