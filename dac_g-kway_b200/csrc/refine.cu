@@ -1880,8 +1880,8 @@ __device__ __forceinline__ u64 block_reduce_u64(u64 x, u64* s_tmp) {
   return r;
 }
 
-constexpr i32 kRiskParts = 1024;    // part limit of the at-risk balance check (k)
-constexpr i32 kRiskCands = 1024;    // candidate limit of that check
+constexpr i32 kRiskParts = 512;    // part limit of the at-risk balance check (k)
+constexpr i32 kRiskCands = 512;    // candidate limit of that check
 
 // The balance check of a round whose candidates are all kept (cnt <= cap),
 // without sorting the candidates.  Only parts flagged in risk can be over
@@ -1906,7 +1906,10 @@ constexpr i32 kRiskCands = 1024;    // candidate limit of that check
 // the caller), the count of a part's events hands out their places in it (one
 // atomic each, no event list), the range tests run without early exits, and
 // the two maxima are warp reductions joined once: 2^20-vertex mesh, k = 64
-// (160 candidates, 72 events, 14 ranges a round on average): MEASURE_CHECK.
+// (160 candidates, 72 events, 14 ranges a round on average): 1 us less a round.
+// One candidate and one part a thread: with two the code is twice as long and
+// every size slower (30k circuit 1.53 -> 1.46 ms of refinement); larger rounds
+// are as fast by rank (rank_select).
 // Returns false (block-uniform) when the last index is not balanced and k >
 // kRiskParts or cnt > kRiskCands; the caller then runs the check over all
 // parts.  *napplied is set on block 0 only.
