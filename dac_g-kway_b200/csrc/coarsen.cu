@@ -658,6 +658,249 @@ void run_group_map(Handle& h, i32 n, const u64* keys, i32 cap, i32* cmap, i32* d
 }
 
 // ===========================================================================
+// Small levels: from the candidates to the contraction's member lists in one
+// launch of one CTA with every table in shared memory -- union-find, group
+// sizes, coarse ids, group orders, member lists, row-length bounds and their
+// scan, the arrays and counters that the row kernels expect cleared.  The
+// separate kernels take thirteen launches and nine clears for this, and on a
+// level of a few thousand vertices each is mostly its launch: the phases here
+// are a chain of shared-memory latencies with a barrier between them.
+// Two levels of a 2048-vertex mesh with k = 8: 186 us with the separate
+// launches, now 134 with the rows and the host's read; a 100k mesh's small
+// levels together 45 us less, a 30k circuit's 55.
+// Per vertex 16 bytes: A parent, then group size | member block << 16, then
+// row length; D distance, then coarse base | members placed << 16, then
+// members; C candidate, then root << 16 | distance, then kPlaced | coarse id;
+// K member keys distance << 16 | id of the groups above the cap, then weight.
+// ===========================================================================
+constexpr int kSmallThreads = 1024;
+constexpr i32 kSmallLevel = 14336;             // 16 bytes each: 224 KB
+constexpr i32 kSmallWarpSort = 1024;           // larger groups are sorted by the whole CTA
+constexpr u32 kPlaced = 0xffff0000u;
+static_assert(kSmallLevel * 16 <= 227 * 1024 - 1024 && kSmallLevel < (1 << 15), "two 16-bit fields a word");
+
+// Ascending sort of a[0..s) in shared memory by lanes [lane0, lane0 + L) of
+// the group that `barrier` waits for.  Every comparison puts the smaller key
+// first, so positions from s to the next power of two act as largest keys
+// that never move and need no storage.
+template <class Barrier>
+__device__ __forceinline__ void sort_in_place(u32* a, i32 s, i32 t, i32 L, Barrier barrier) {
+  i32 P = 2;
+  while (P < s) P <<= 1;
+  for (i32 kk = 2; kk <= P; kk <<= 1) {
+    for (i32 j = kk >> 1; j > 0; j >>= 1) {
+      const bool mirror = 2 * j == kk;   // the first step of a merge pairs i with its mirror in the block
+      for (i32 q = t; q < P / 2; q += L) {
+        const i32 i = 2 * (q & ~(j - 1)) | (q & (j - 1));
+        const i32 l = mirror ? (i ^ (kk - 1)) : (i | j);
+        if (l < s) {
+          const u32 x = a[i], y = a[l];
+          if (x > y) {
+            a[i] = y;
+            a[l] = x;
+          }
+        }
+      }
+      barrier();
+    }
+  }
+}
+
+// Exclusive scan of x[0..n) (0 <= i < n) by the CTA: each warp a contiguous
+// segment, `value(i)` a word, `store(i, exclusive, value)`; returns the total.
+// s_warp has one word per warp.  Starts and ends with a barrier.
+template <class Value, class Store>
+__device__ __forceinline__ u32 scan_segments(i32 n, u32* s_warp, Value value, Store store) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const i32 seg = (((n + warps - 1) / warps) + 31) & ~31;
+  const i32 b = warp * seg < n ? warp * seg : n, e = b + seg < n ? b + seg : n;
+  __syncthreads();
+  u32 sum = 0;
+  for (i32 i = b + lane; i < e; i += 32) sum += value(i);
+  sum = __reduce_add_sync(kFull, sum);
+  if (lane == 0) s_warp[warp] = sum;
+  __syncthreads();
+  u32 w = lane < warps ? s_warp[lane] : 0;
+  const u32 total = __reduce_add_sync(kFull, w);
+  u32 run = __reduce_add_sync(kFull, lane < warp ? w : 0);
+  for (i32 i0 = b; i0 < e; i0 += 32) {
+    const i32 i = i0 + lane;
+    const u32 x = i < e ? value(i) : 0;
+    u32 inc = x;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const u32 y = __shfl_up_sync(kFull, inc, o);
+      if (lane >= o) inc += y;
+    }
+    if (i < e) store(i, run + inc - x, x);
+    run += __shfl_sync(kFull, inc, 31);
+  }
+  __syncthreads();
+  return total;
+}
+
+struct SmallLevel {
+  i32 n, cap;
+  const i32* cand;
+  const i32 *xadj, *vwgt;
+  i32 *cmap, *cvwgt, *rowlen, *ub, *mcnt, *memtab, *cnt, *misc;
+  ArenaHdr* arena;
+  i32 *nc, *uf_rounds, *max_cvw, *maxdeg;
+};
+
+__global__ void __launch_bounds__(kSmallThreads) k_group_small(SmallLevel a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ u32 s_warp[kSmallThreads / 32];
+  __shared__ i32 s_rounds;
+  const i32 n = a.n, cap = a.cap, T = (i32)blockDim.x, t = (i32)threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  u32* A = reinterpret_cast<u32*>(smem_raw);
+  u32* D = A + n;
+  u32* C = D + n;
+  u32* K = C + n;
+  i32* parent = reinterpret_cast<i32*>(A);
+  i32* cand = reinterpret_cast<i32*>(C);
+  for (i32 v = t; v < n; v += T) {
+    const i32 c = a.cand[v];
+    cand[v] = c;
+    parent[v] = c > v ? c : v;
+    D[v] = kUfUnknown;
+  }
+  if (t == 0) s_rounds = 0;
+  if (t < 8) a.misc[t] = 0;
+  if (t == 0) {
+    a.arena->used = 0;
+    a.arena->need = 0;
+    a.arena->overflow = 0;
+    *a.max_cvw = 0;
+    *a.maxdeg = 0;
+  }
+  __syncthreads();
+  for (i32 v = t; v < n; v += T)
+    if (cand[v] < v) uf_unite<true>(parent, v, cand[v]);
+  __syncthreads();
+  for (i32 v = t; v < n; v += T)
+    if (parent[v] == v) uf_mark_root<true>(cand, D, v);
+  __syncthreads();
+  u32 far = 0;
+  for (i32 v = t; v < n; v += T) {
+    const u32 d = uf_walk<true>(cand, D, v);
+    *(volatile u32*)(D + v) = d;
+    far = d > far ? d : far;
+  }
+  uf_max_rounds(far, &s_rounds);
+  __syncthreads();
+  for (i32 v = t; v < n; v += T) C[v] = ((u32)uf_find<true>(parent, v) << 16) | D[v];
+  __syncthreads();
+  for (i32 v = t; v < n; v += T) A[v] = 0;
+  __syncthreads();
+  for (i32 v = t; v < n; v += T) atomicAdd(&A[C[v] >> 16], 1u);
+  // coarse ids in root order, and the member blocks of the groups above the cap
+  const u32 sums = scan_segments(
+      n, s_warp,
+      [&](i32 v) {
+        const u32 s = A[v] & 0xffffu;
+        return (s + (u32)cap - 1) / (u32)cap | (s > (u32)cap ? s << 16 : 0u);
+      },
+      [&](i32 v, u32 before, u32) {
+        D[v] = before & 0xffffu;
+        A[v] |= before & 0xffff0000u;
+      });
+  const i32 nc = (i32)(sums & 0xffffu);
+  for (i32 v = t; v < n; v += T) {
+    const u32 key = C[v], r = key >> 16, sz = A[r];
+    if ((sz & 0xffffu) <= (u32)cap) {
+      C[v] = kPlaced | (D[r] & 0xffffu);
+    } else {
+      const u32 slot = atomicAdd(&D[r], 1u << 16) >> 16;
+      K[(sz >> 16) + slot] = (key << 16) | (u32)v;
+    }
+  }
+  __syncthreads();
+  if (sums >> 16) {   // groups above the cap: members in (distance, id) order
+    bool large = false;
+    for (i32 v0 = t - lane; v0 < n; v0 += T) {
+      const i32 v = v0 + lane;
+      const u32 s = v < n && C[v] >> 16 == (u32)v ? A[v] & 0xffffu : 0;
+      large |= s > (u32)kSmallWarpSort;
+      u32 todo = __ballot_sync(kFull, s > 0 && s <= (u32)kSmallWarpSort);   // (placed vertices are no roots)
+      while (todo) {
+        const int q = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const u32 w = A[v0 + q], base = D[v0 + q] & 0xffffu;
+        const i32 m = (i32)(w & 0xffffu);
+        u32* k = K + (w >> 16);
+        __syncwarp();
+        if (m <= 32) {
+          u32 key = lane < m ? k[lane] : ~0u;
+#pragma unroll
+          for (int kk = 2; kk <= 32; kk <<= 1) {
+#pragma unroll
+            for (int j = kk >> 1; j > 0; j >>= 1) {
+              const u32 o = __shfl_xor_sync(kFull, key, j);
+              const bool low = ((lane & kk) == 0) == ((lane & j) == 0);
+              key = low ? min(key, o) : max(key, o);
+            }
+          }
+          if (lane < m) C[key & 0xffffu] = kPlaced | (base + (u32)(lane / cap));
+        } else {
+          sort_in_place(k, m, lane, 32, [] { __syncwarp(); });
+          for (i32 i = lane; i < m; i += 32) C[k[i] & 0xffffu] = kPlaced | (base + (u32)(i / cap));
+        }
+        __syncwarp();
+      }
+    }
+    const bool any = __syncthreads_or(large);
+    for (i32 v0 = 0; any && v0 < n; v0 += T) {   // at most n / kSmallWarpSort groups
+      const i32 v = v0 + t;
+      const bool big = v < n && C[v] >> 16 == (u32)v;
+      while (true) {
+        const i32 mine = big && C[v] >> 16 == (u32)v ? v : -1;
+        if (t == 0) s_warp[0] = 0;
+        __syncthreads();
+        if (mine >= 0) atomicMax(&s_warp[0], (u32)mine + 1u);
+        __syncthreads();
+        const i32 r = (i32)s_warp[0] - 1;
+        __syncthreads();
+        if (r < 0) break;
+        const u32 w = A[r], base = D[r] & 0xffffu;
+        const i32 m = (i32)(w & 0xffffu);
+        u32* k = K + (w >> 16);
+        sort_in_place(k, m, t, T, [] { __syncthreads(); });
+        for (i32 i = t; i < m; i += T) C[k[i] & 0xffffu] = kPlaced | (base + (u32)(i / cap));
+        __syncthreads();
+      }
+    }
+  }
+  // member lists, row-length bounds and weights of the coarse vertices
+  for (i32 c = t; c < nc; c += T) A[c] = D[c] = K[c] = 0;
+  __syncthreads();
+#pragma unroll 4
+  for (i32 v = t; v < n; v += T) {
+    const u32 c = C[v] & 0xffffu;
+    const i32 len = __ldg(a.xadj + v + 1) - __ldg(a.xadj + v);
+    const u32 w = (u32)__ldg(a.vwgt + v);
+    a.cmap[v] = (i32)c;
+    atomicAdd(&A[c], (u32)len);
+    atomicAdd(&K[c], w);
+    a.memtab[(i64)c * cap + (i32)atomicAdd(&D[c], 1u)] = v;
+  }
+  scan_segments(
+      nc, s_warp, [&](i32 c) { return A[c]; },
+      [&](i32 c, u32 before, u32 len) {
+        a.rowlen[c] = (i32)len;
+        a.ub[c] = (i32)before;
+        a.mcnt[c] = (i32)D[c];
+        a.cvwgt[c] = (i32)K[c];
+      });
+  for (i32 c = t; c <= n; c += T) a.cnt[c] = 0;   // rows from n_c on are empty
+  if (t == 0) {
+    *a.nc = nc;
+    *a.uf_rounds = s_rounds;
+  }
+}
+
+// ===========================================================================
 // Contraction (coarsen.hpp:157-349).  Members of each coarse vertex are
 // listed (at most group_cap of them); then one warp per coarse vertex hashes
 // the mapped neighbour ids of all its members into shared memory, summing
@@ -1288,32 +1531,93 @@ void ensure_arena(Handle& h, u64 words) {
   h.arena_words = words;
 }
 
+// The tables that the row kernels share.
+struct ContractTables {
+  i32 *rowlen, *ub, *mcnt, *memtab, *cnt, *heavy, *mid;
+  i32* misc;   // [0] heavy rows, [1] ub total, [2] rows listed by the short kernel
+  i32 *sadj, *swgt;
+};
+
+static ContractTables contract_tables(Handle& h, i64 m, i32 nc_ub, i32 cap) {
+  const i64 nu = (i64)nc_ub + 1;
+  ContractTables t;
+  t.rowlen = h.scratch.alloc_n<i32>(nu);
+  t.ub = h.scratch.alloc_n<i32>(nu);
+  t.mcnt = h.scratch.alloc_n<i32>(nu);
+  t.memtab = h.scratch.alloc_n<i32>((i64)nc_ub * cap + 1);
+  t.cnt = h.scratch.alloc_n<i32>(nu);
+  t.heavy = h.scratch.alloc_n<i32>(nu);
+  t.mid = h.scratch.alloc_n<i32>(nu);
+  t.misc = h.scratch.alloc_n<i32>(8);
+  t.sadj = h.scratch.alloc_n<i32>(std::max<i64>(m, 1));
+  t.swgt = h.scratch.alloc_n<i32>(std::max<i64>(m, 1));
+  return t;
+}
+
+static void contract_rows(Handle& h, const DevGraph& g, const ContractTables& t, const i32* cmap, const i32* d_nc,
+                          i32 nc_ub, i32 cap, i32* cxadj, i32* cadjncy, i32* cadjwgt, const i32* cvwgt, i32* d_mc);
+
 void run_contract(Handle& h, const DevGraph& g, const i32* cmap, const i32* d_nc, i32 nc_ub, i32 cap, i32* cxadj,
                   i32* cadjncy, i32* cadjwgt, i32* cvwgt, i32* d_mc) {
   Pool::Mark mk = h.scratch.mark();
   const i32 n = g.n;
   const i64 nu = (i64)nc_ub + 1;
   const u32 nb = ceil_div(std::max(n, 1), 256);
-  i32* rowlen = h.scratch.alloc_n<i32>(nu);
-  i32* ub = h.scratch.alloc_n<i32>(nu);
-  i32* mcnt = h.scratch.alloc_n<i32>(nu);
-  i32* memtab = h.scratch.alloc_n<i32>((i64)nc_ub * cap + 1);
-  i32* cnt = h.scratch.alloc_n<i32>(nu);
-  i32* heavy = h.scratch.alloc_n<i32>(nu);
-  i32* mid = h.scratch.alloc_n<i32>(nu);
-  i32* misc = h.scratch.alloc_n<i32>(8);   // [0] heavy rows, [1] ub total, [2] rows listed by the short kernel
-  i32* sadj = h.scratch.alloc_n<i32>(std::max<i64>(g.m, 1));
-  i32* swgt = h.scratch.alloc_n<i32>(std::max<i64>(g.m, 1));
+  const ContractTables t = contract_tables(h, g.m, nc_ub, cap);
   ensure_arena(h, u64(4) << 20);   // 16 MB of long-row tables to start with
   GKW_CUDA(cudaMemsetAsync(cvwgt, 0, sizeof(i32) * std::max(nc_ub, 1), h.stream));
-  GKW_CUDA(cudaMemsetAsync(rowlen, 0, sizeof(i32) * nu, h.stream));
-  GKW_CUDA(cudaMemsetAsync(mcnt, 0, sizeof(i32) * nu, h.stream));
-  GKW_CUDA(cudaMemsetAsync(cnt, 0, sizeof(i32) * nu, h.stream));
-  GKW_CUDA(cudaMemsetAsync(misc, 0, sizeof(i32) * 8, h.stream));
+  GKW_CUDA(cudaMemsetAsync(t.rowlen, 0, sizeof(i32) * nu, h.stream));
+  GKW_CUDA(cudaMemsetAsync(t.mcnt, 0, sizeof(i32) * nu, h.stream));
+  GKW_CUDA(cudaMemsetAsync(t.cnt, 0, sizeof(i32) * nu, h.stream));
+  GKW_CUDA(cudaMemsetAsync(t.misc, 0, sizeof(i32) * 8, h.stream));
   if (n > 0)
-    launch(k_coarse_accum, nb, 256, 0, h.stream, n, g.xadj, g.vwgt, cmap, cap, cvwgt, rowlen, mcnt, memtab, h.arena);
+    launch(k_coarse_accum, nb, 256, 0, h.stream, n, g.xadj, g.vwgt, cmap, cap, cvwgt, t.rowlen, t.mcnt, t.memtab,
+           h.arena);
   GKW_CHECK_LAUNCH();
-  exclusive_scan_i32(h, rowlen, ub, nu, misc + 1);   // rows beyond n_c have length 0
+  exclusive_scan_i32(h, t.rowlen, t.ub, nu, t.misc + 1);   // rows beyond n_c have length 0
+  contract_rows(h, g, t, cmap, d_nc, nc_ub, cap, cxadj, cadjncy, cadjwgt, cvwgt, d_mc);
+  h.scratch.release(mk);
+}
+
+// A level of at most kSmallLevel vertices from its candidates on.
+static void run_small_level(Handle& h, const DevGraph& g, const i32* cand, i32 cap, const CoarsenOut& out) {
+  Pool::Mark mk = h.scratch.mark();
+  const ContractTables t = contract_tables(h, g.m, g.n, cap);
+  SmallLevel a;
+  a.n = g.n;
+  a.cap = cap;
+  a.cand = cand;
+  a.xadj = g.xadj;
+  a.vwgt = g.vwgt;
+  a.cmap = out.cmap;
+  a.cvwgt = out.cvwgt;
+  a.rowlen = t.rowlen;
+  a.ub = t.ub;
+  a.mcnt = t.mcnt;
+  a.memtab = t.memtab;
+  a.cnt = t.cnt;
+  a.misc = t.misc;
+  a.arena = h.arena;
+  a.nc = &h.coop->nc;
+  a.uf_rounds = &h.coop->uf_rounds;
+  a.max_cvw = &h.coop->max_cvw;
+  a.maxdeg = &h.coop->maxdeg;
+  if (!h.capturing)
+    GKW_CUDA(cudaFuncSetAttribute(k_group_small, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallLevel * 16));
+  launch(k_group_small, 1, kSmallThreads, (size_t)g.n * 16, h.stream, a);
+  GKW_CHECK_LAUNCH();
+  contract_rows(h, g, t, out.cmap, &h.coop->nc, g.n, cap, out.cxadj, out.cadjncy, out.cadjwgt, out.cvwgt,
+                &h.coop->mc);
+  h.scratch.release(mk);
+}
+
+// The coarse rows from the prepared tables.
+static void contract_rows(Handle& h, const DevGraph& g, const ContractTables& t, const i32* cmap, const i32* d_nc,
+                          i32 nc_ub, i32 cap, i32* cxadj, i32* cadjncy, i32* cadjwgt, const i32* cvwgt, i32* d_mc) {
+  const i32 n = g.n;
+  const i64 nu = (i64)nc_ub + 1;
+  i32 *const rowlen = t.rowlen, *const ub = t.ub, *const mcnt = t.mcnt, *const memtab = t.memtab, *const cnt = t.cnt;
+  i32 *const heavy = t.heavy, *const mid = t.mid, *const misc = t.misc, *const sadj = t.sadj, *const swgt = t.swgt;
   // Expected coarse row: a group's members (about five; at most cap) times the
   // mean degree.  Short rows take 16 lanes each (12M-vertex road graph, 7
   // entries a row: 3.2 ms with a warp each, now 1.4 over all levels); else one
@@ -1377,9 +1681,8 @@ void run_contract(Handle& h, const DevGraph& g, const i32* cmap, const i32* d_nc
   const i32 R = expL > 200 ? 1 : nc_ub > 100000 ? 32 : expL <= 48 ? 8 : 4;
   if (nc_ub > 0)
     launch(k_copy_rows, std::min<u32>(ceil_div((u64)nc_ub, 8 * (u64)R), (u32)h.sm_count * 32), 256, 0, h.stream, d_nc, R, ub, cnt, cxadj, sadj, swgt, cadjncy,
-           cadjwgt, &h.coop->maxdeg, (const i32*)cvwgt, &h.coop->max_cvw);
+           cadjwgt, &h.coop->maxdeg, cvwgt, &h.coop->max_cvw);
   GKW_CHECK_LAUNCH();
-  h.scratch.release(mk);
 }
 
 CoopState read_coop(Handle& h) {
@@ -2318,6 +2621,11 @@ void coarsen_level(Handle& h, const DevGraph& g, i32 cap, CoarsenOut& out) {
     u64* keys = h.scratch.alloc_n<u64>(std::max(g.n, 1));
     if (tune) time_match_variants(h, g, cand);
     run_match(h, g, cand, g.maxdeg);
+    if (g.n > 0 && g.n <= kSmallLevel) {
+      run_small_level(h, g, cand, cap, out);
+      h.scratch.release(mk);
+      return;
+    }
     run_union_find(h, g.n, cand, keys, &h.coop->uf_rounds);
     run_group_map(h, g.n, keys, cap, out.cmap, &h.coop->nc);
     h.scratch.release(mk);
