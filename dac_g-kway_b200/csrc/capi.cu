@@ -130,7 +130,7 @@ gkw_status gkw_create(gkw_handle** out, int32_t device) {
     h->h.own_stream = true;
     // GKW_GRAPHS=0: launch sequences always run as is (no CUDA-graph replay)
     if (const char* gs = getenv("GKW_GRAPHS")) h->h.graphs_on = *gs != '0';
-    e = cudaMallocHost(&h->h.h_pinned, 64 * sizeof(int64_t));
+    e = cudaMallocHost(&h->h.h_pinned, kPinnedWords * sizeof(int64_t));
     if (e != cudaSuccess) {
       cudaStreamDestroy(h->h.stream);
       delete h;

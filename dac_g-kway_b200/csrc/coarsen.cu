@@ -617,19 +617,18 @@ void run_group_map(Handle& h, i32 n, const u64* keys, i32 cap, i32* cmap, i32* d
   }
   Pool::Mark mk = h.scratch.mark();
   const u32 nb = ceil_div(n, 256);
-  i32* gsize = h.scratch.alloc_n<i32>(n);
+  const size_t nz = ((size_t)n + 63) & ~(size_t)63;
+  i32* gsize = h.scratch.alloc_n<i32>(2 * nz + 8);   // cleared together with gcur and counts
+  i32* gcur = gsize + nz;
+  i32* counts = gcur + nz;
   i32* chunks = h.scratch.alloc_n<i32>(n);
   i32* bigsz = h.scratch.alloc_n<i32>(n);
-  i32* gcur = h.scratch.alloc_n<i32>(n);
   i32* members = h.scratch.alloc_n<i32>(n);
   i32* biglist = h.scratch.alloc_n<i32>(n);
   i32* giantlist = h.scratch.alloc_n<i32>(n);
   i32* ctalist = h.scratch.alloc_n<i32>(n);
-  i32* counts = h.scratch.alloc_n<i32>(8);
   u64* gscratch = h.scratch.alloc_n<u64>(2 * (size_t)n);
-  GKW_CUDA(cudaMemsetAsync(gsize, 0, sizeof(i32) * n, h.stream));
-  GKW_CUDA(cudaMemsetAsync(gcur, 0, sizeof(i32) * n, h.stream));
-  GKW_CUDA(cudaMemsetAsync(counts, 0, sizeof(i32) * 8, h.stream));
+  GKW_CUDA(cudaMemsetAsync(gsize, 0, sizeof(i32) * (2 * nz + 8), h.stream));
   launch(k_group_count, nb, 256, 0, h.stream, n, keys, gsize);
   launch(k_group_chunks, nb, 256, 0, h.stream, n, gsize, cap, chunks, bigsz, counts + 3);
   GKW_CHECK_LAUNCH();
@@ -913,12 +912,16 @@ __global__ void __launch_bounds__(kSmallThreads) k_group_small(SmallLevel a) {
 __global__ void k_coarse_accum(i32 n, const i32* __restrict__ xadj, const i32* __restrict__ vwgt,
                                const i32* __restrict__ cmap, i32 cap, i32* __restrict__ cvwgt,
                                i32* __restrict__ rowlen, i32* __restrict__ mcnt, i32* __restrict__ memtab,
-                               ArenaHdr* arena) {
+                               ArenaHdr* arena, CoopState* coop) {
   const i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-  if (v == 0 && arena) {
-    arena->used = 0;
-    arena->need = 0;
-    arena->overflow = 0;
+  if (v == 0) {
+    if (arena) {
+      arena->used = 0;
+      arena->need = 0;
+      arena->overflow = 0;
+    }
+    coop->max_cvw = 0;
+    coop->maxdeg = 0;
   }
   if (v >= n) return;
   const i32 c = cmap[v];
@@ -1536,19 +1539,21 @@ struct ContractTables {
   i32 *rowlen, *ub, *mcnt, *memtab, *cnt, *heavy, *mid;
   i32* misc;   // [0] heavy rows, [1] ub total, [2] rows listed by the short kernel
   i32 *sadj, *swgt;
+  size_t nz;
 };
 
 static ContractTables contract_tables(Handle& h, i64 m, i32 nc_ub, i32 cap) {
   const i64 nu = (i64)nc_ub + 1;
   ContractTables t;
-  t.rowlen = h.scratch.alloc_n<i32>(nu);
+  t.nz = ((size_t)nu + 63) & ~(size_t)63;
+  t.rowlen = h.scratch.alloc_n<i32>(3 * t.nz + 8);   // cleared together: rowlen, mcnt, cnt, misc
+  t.mcnt = t.rowlen + t.nz;
+  t.cnt = t.mcnt + t.nz;
+  t.misc = t.cnt + t.nz;
   t.ub = h.scratch.alloc_n<i32>(nu);
-  t.mcnt = h.scratch.alloc_n<i32>(nu);
   t.memtab = h.scratch.alloc_n<i32>((i64)nc_ub * cap + 1);
-  t.cnt = h.scratch.alloc_n<i32>(nu);
   t.heavy = h.scratch.alloc_n<i32>(nu);
   t.mid = h.scratch.alloc_n<i32>(nu);
-  t.misc = h.scratch.alloc_n<i32>(8);
   t.sadj = h.scratch.alloc_n<i32>(std::max<i64>(m, 1));
   t.swgt = h.scratch.alloc_n<i32>(std::max<i64>(m, 1));
   return t;
@@ -1566,13 +1571,12 @@ void run_contract(Handle& h, const DevGraph& g, const i32* cmap, const i32* d_nc
   const ContractTables t = contract_tables(h, g.m, nc_ub, cap);
   ensure_arena(h, u64(4) << 20);   // 16 MB of long-row tables to start with
   GKW_CUDA(cudaMemsetAsync(cvwgt, 0, sizeof(i32) * std::max(nc_ub, 1), h.stream));
-  GKW_CUDA(cudaMemsetAsync(t.rowlen, 0, sizeof(i32) * nu, h.stream));
-  GKW_CUDA(cudaMemsetAsync(t.mcnt, 0, sizeof(i32) * nu, h.stream));
-  GKW_CUDA(cudaMemsetAsync(t.cnt, 0, sizeof(i32) * nu, h.stream));
-  GKW_CUDA(cudaMemsetAsync(t.misc, 0, sizeof(i32) * 8, h.stream));
+  GKW_CUDA(cudaMemsetAsync(t.rowlen, 0, sizeof(i32) * (3 * t.nz + 8), h.stream));
   if (n > 0)
     launch(k_coarse_accum, nb, 256, 0, h.stream, n, g.xadj, g.vwgt, cmap, cap, cvwgt, t.rowlen, t.mcnt, t.memtab,
-           h.arena);
+           h.arena, h.coop);
+  else   // (two words)
+    GKW_CUDA(cudaMemsetAsync(&h.coop->max_cvw, 0, 2 * sizeof(i32), h.stream));
   GKW_CHECK_LAUNCH();
   exclusive_scan_i32(h, t.rowlen, t.ub, nu, t.misc + 1);   // rows beyond n_c have length 0
   contract_rows(h, g, t, cmap, d_nc, nc_ub, cap, cxadj, cadjncy, cadjwgt, cvwgt, d_mc);
@@ -1685,15 +1689,34 @@ static void contract_rows(Handle& h, const DevGraph& g, const ContractTables& t,
   GKW_CHECK_LAUNCH();
 }
 
-CoopState read_coop(Handle& h) {
-  CoopState* hc = reinterpret_cast<CoopState*>(h.h_pinned);
-  static_assert(sizeof(CoopState) + sizeof(ArenaHdr) + 8 <= 64 * sizeof(i64), "pinned staging too small");
-  GKW_CUDA(cudaMemcpyAsync(hc, h.coop, sizeof(CoopState), cudaMemcpyDeviceToHost, h.stream));
-  ArenaHdr* ha = reinterpret_cast<ArenaHdr*>(hc + 1);
-  if (h.arena) GKW_CUDA(cudaMemcpyAsync(ha, h.arena, sizeof(ArenaHdr), cudaMemcpyDeviceToHost, h.stream));
-  i32* hs = reinterpret_cast<i32*>(ha + 1);
-  if (h.scan) GKW_CUDA(cudaMemcpyAsync(hs, &h.scan->err, sizeof(i32), cudaMemcpyDeviceToHost, h.stream));
+// The level's scalars and error words straight into the handle's pinned words.
+struct CoopReport {
+  CoopState coop;
+  ArenaHdr arena;
+  i32 scan_err;
+};
+static_assert(sizeof(CoopReport) <= kPinnedWords * sizeof(i64), "pinned words too few");
+
+__global__ void k_coop_report(const CoopState* coop, const ArenaHdr* arena, const ScanState* scan, CoopReport* out) {
+  out->coop = *coop;
+  if (arena) out->arena = *arena;
+  out->scan_err = scan ? scan->err : 0;
+}
+
+static void report_coop(Handle& h) {
+  launch(k_coop_report, 1, 1, 0, h.stream, (const CoopState*)h.coop, (const ArenaHdr*)h.arena,
+         (const ScanState*)h.scan, reinterpret_cast<CoopReport*>(h.h_pinned));
+  GKW_CHECK_LAUNCH();
+}
+
+// reported: the stream's last launch was report_coop
+CoopState read_coop(Handle& h, bool reported) {
+  if (!reported) report_coop(h);
   GKW_CUDA(cudaStreamSynchronize(h.stream));
+  const CoopReport* r = reinterpret_cast<const CoopReport*>(h.h_pinned);
+  const CoopState* hc = &r->coop;
+  const ArenaHdr* ha = &r->arena;
+  const i32* hs = &r->scan_err;
   CoopState c = *hc;
   c.arena_overflow = h.arena ? ha->overflow : 0;
   c.arena_need = h.arena ? (i64)ha->need : 0;
@@ -2629,24 +2652,25 @@ void coarsen_level(Handle& h, const DevGraph& g, i32 cap, CoarsenOut& out) {
     run_union_find(h, g.n, cand, keys, &h.coop->uf_rounds);
     run_group_map(h, g.n, keys, cap, out.cmap, &h.coop->nc);
     h.scratch.release(mk);
-    static_assert(offsetof(CoopState, maxdeg) == offsetof(CoopState, max_cvw) + sizeof(i32),
-                  "max_cvw and maxdeg are cleared together");
-    GKW_CUDA(cudaMemsetAsync(&h.coop->max_cvw, 0, 2 * sizeof(i32), h.stream));
     run_contract(h, g, out.cmap, &h.coop->nc, g.n, cap, out.cxadj, out.cadjncy, out.cadjwgt, out.cvwgt,
                  &h.coop->mc);
   };
+  bool reported = false;
   if (use_fused(h, g)) {
     // one launch: no graph needed (a launch is as cheap as a graph of one)
     run_coarsen_fused(h, g, cap, out);
   } else if (tune) {
     body();   // the tuner's timings synchronise: never captured
   } else {
-    graph_run(h, level_key(h, g, cap, out), body);
+    graph_run(h, level_key(h, g, cap, out), [&] {
+      body();
+      report_coop(h);
+    });
+    reported = true;
   }
-  CoopState c = read_coop(h);
+  CoopState c = read_coop(h, reported);
   if (c.arena_overflow) {   // very long coarse rows: grow the arena and redo the step
     ensure_arena(h, (u64)((double)(h.arena_words + (u64)c.arena_need) * 1.25) + 1024);
-    GKW_CUDA(cudaMemsetAsync(&h.coop->maxdeg, 0, sizeof(i32), h.stream));
     run_contract(h, g, out.cmap, &h.coop->nc, g.n, cap, out.cxadj, out.cadjncy, out.cadjwgt, out.cvwgt,
                  &h.coop->mc);
     c = read_coop(h);

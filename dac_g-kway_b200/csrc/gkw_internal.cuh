@@ -132,6 +132,8 @@ struct CountBarrier {
   unsigned long long w[3];
 };
 
+constexpr int kPinnedWords = 1024;   // Handle::h_pinned
+
 // Device-side state of one handle shared by the cooperative kernels and the
 // per-level scalars read back once per level.
 struct CoopState {
@@ -306,7 +308,7 @@ void run_contract(Handle& h, const DevGraph& g, const i32* cmap, const i32* d_nc
                   i32* cxadj, i32* cadjncy, i32* cadjwgt, i32* cvwgt, i32* d_mc);
 void ensure_arena(Handle& h, u64 words);
 // Reads the CoopState (one host sync) and throws on a recorded error.
-CoopState read_coop(Handle& h);
+CoopState read_coop(Handle& h, bool reported = false);
 void coarsen_level(Handle& h, const DevGraph& g, i32 group_cap, CoarsenOut& out);
 
 // ---- refinement (refine.cu) ----
@@ -375,14 +377,24 @@ void refine_init_union(Handle& h, RefineCtx* c, const DevGraph& cu, const i32* p
 void level_run(Handle& h, RefineCtx* c, const DevGraph& g, const LevelJob& j, i32 stats_slot);
 // Reads the per-level statistics of slots [0, nslots) (one host sync); throws
 // if a level kernel reported an error.
-std::vector<RefineLevelStats> level_stats(Handle& h, RefineCtx* c, i32 nslots);
+// One sync: the slots' statistics; throws on an error word of the level
+// kernels.  metrics: d_metrics (compute_cut_pw) and d_init (or null) in, the
+// rest out.
+struct RunMetrics {
+  const i64* d_metrics = nullptr;
+  const i64* d_init = nullptr;
+  i64 cut = 0, bad = 0, max_pw = 0, init_cut = 0;
+};
+std::vector<RefineLevelStats> level_stats(Handle& h, RefineCtx* c, i32 nslots, RunMetrics* metrics = nullptr);
 // (1 + eps) * W / k, the default-mode weight cap (no "+1").
 float balance_cap(i64 total_vwgt, i32 k, double eps);
 
 // ---- metrics (refine.cu) ----
 // d_cut needs 2 slots ([0] cut, [1] nonzero if a part id was out of range);
 // d_pw needs k.
-void compute_cut_pw(Handle& h, const DevGraph& g, const i32* part, i32 k, i64* d_cut, i64* d_pw);
+// cleared: the k + 2 words are zero already
+void compute_cut_pw(Handle& h, const DevGraph& g, const i32* part, i32 k, i64* d_cut, i64* d_pw,
+                    bool cleared = false);
 // The cut / part-weight kernel alone: d_acc[0] cut, [1] bad-part flag,
 // [2..k+2) part weights; the caller zeroes d_acc first.
 void launch_cut_pw(cudaStream_t stream, i32 sm_count, const DevGraph& g, const i32* part, i32 k, i64* d_acc);

@@ -125,26 +125,24 @@ __global__ void k_sub_i32(i32* p, i64 n, i32 v) {
 // returns total vertex weight (the longest row in *maxdeg); throws on malformed input
 i64 validate(Handle& h, const DevGraph& g, i64* maxdeg) {
   Pool::Mark mk = h.scratch.mark();
-  i32* flags = h.scratch.alloc_n<i32>(4);   // [0] error bits, [1] longest row, [2] long rows
-  unsigned long long* ws = h.scratch.alloc_n<unsigned long long>(1);
+  i32* flags = h.scratch.alloc_n<i32>(6);   // [0] error bits, [1] longest row, [2] (64 bits) weight, [4] long rows
+  unsigned long long* ws = reinterpret_cast<unsigned long long*>(flags + 2);
   i32* longlist = h.scratch.alloc_n<i32>(std::max(g.n, 1));
-  GKW_CUDA(cudaMemsetAsync(flags, 0, sizeof(i32) * 4, h.stream));
-  GKW_CUDA(cudaMemsetAsync(ws, 0, sizeof(u64), h.stream));
+  GKW_CUDA(cudaMemsetAsync(flags, 0, sizeof(i32) * 6, h.stream));
   if (g.n > 0) {
     const double avg = (double)g.m / g.n;
     auto go = [&](auto kern, int G) {
       launch(kern, ceil_div((u64)g.n * G, 256), 256, 0, h.stream, g.n, g.m, g.xadj, g.adjncy, g.adjwgt, g.vwgt,
-             flags, ws, longlist, flags + 2);
+             flags, ws, longlist, flags + 4);
     };
     if (avg <= 6.5) go(k_validate<4>, 4);
     else if (avg <= 14) go(k_validate<8>, 8);
     else go(k_validate<16>, 16);
     launch(k_validate_long, (u32)h.sm_count * 2, 256, 0, h.stream, g.n, g.xadj, g.adjncy, g.adjwgt, flags,
-           (const i32*)longlist, (const i32*)(flags + 2));
+           (const i32*)longlist, (const i32*)(flags + 4));
     GKW_CHECK_LAUNCH();
   }
-  GKW_CUDA(cudaMemcpyAsync(h.h_pinned, flags, sizeof(i32) * 2, cudaMemcpyDeviceToHost, h.stream));
-  GKW_CUDA(cudaMemcpyAsync(h.h_pinned + 1, ws, sizeof(u64), cudaMemcpyDeviceToHost, h.stream));
+  GKW_CUDA(cudaMemcpyAsync(h.h_pinned, flags, sizeof(i32) * 4, cudaMemcpyDeviceToHost, h.stream));
   GKW_CUDA(cudaStreamSynchronize(h.stream));
   const i32 f = (i32)(h.h_pinned[0] & 0xffffffff);
   if (maxdeg) *maxdeg = (i32)((u64)h.h_pinned[0] >> 32);
@@ -292,10 +290,11 @@ void partition_impl(Handle& h, const DevGraph& g0, i32 k, const gkw_options& opt
   initial_partition(h, cg, k, opt, cpart);
   if (stage_checks()) check_stage("initial partition", (i32)lv.size() - 1, [&] { check_parts(h, cg.n, cpart, k); });
   refine_init_coarsest(h, rc, cg, cpart);
-  i64* d_metrics = h.hier.alloc_n<i64>(k + 2);   // [0] cut, [1] bad-part flag, [2..k+2) part weights
-  i64* d_init = h.hier.alloc_n<i64>(k + 2);      // the same for the initial partition
+  i64* d_metrics = h.hier.alloc_n<i64>(2 * ((size_t)k + 2));   // [0] cut, [1] bad-part flag, [2..k+2) part weights
+  i64* d_init = d_metrics + k + 2;                             // the same for the initial partition
+  GKW_CUDA(cudaMemsetAsync(d_metrics, 0, sizeof(i64) * 2 * ((size_t)k + 2), h.stream));
   if (stats)   // cut of the initial partition itself (before any balance move), read at the end
-    compute_cut_pw(h, cg, refine_part(rc), k, d_init, d_init + 2);
+    compute_cut_pw(h, cg, refine_part(rc), k, d_init, d_init + 2, true);
   const i32 nl = (i32)lv.size();
   // default mode: balance rounds at every level but the balance_skip_levels
   // coarsest ones (the finest level always)
@@ -333,16 +332,15 @@ void partition_impl(Handle& h, const DevGraph& g0, i32 k, const gkw_options& opt
     GKW_CUDA(cudaMemcpyAsync(d_part_out, refine_part(rc), sizeof(i32) * g0.n, cudaMemcpyDeviceToDevice,
                              h.stream));
   }
-  compute_cut_pw(h, g0, d_part_out, k, d_metrics, d_metrics + 2);
-  std::vector<i64> hm(k + 2);
-  GKW_CUDA(cudaMemcpyAsync(hm.data(), d_metrics, sizeof(i64) * (k + 2), cudaMemcpyDeviceToHost, h.stream));
-  i64 init_cut = 0;
-  if (stats) GKW_CUDA(cudaMemcpyAsync(&init_cut, d_init, sizeof(i64), cudaMemcpyDeviceToHost, h.stream));
+  compute_cut_pw(h, g0, d_part_out, k, d_metrics, d_metrics + 2, true);
   GKW_CUDA(cudaEventRecord(ev[4], h.stream));
   // one host sync for the statistics, the error words and the metrics above
-  std::vector<RefineLevelStats> rs = level_stats(h, rc, nl);
-  GKW_REQUIRE(hm[1] == 0, GKW_E_INTERNAL, "partition produced a part id out of range");
-  if (cut_out) *cut_out = hm[0];
+  RunMetrics rm;
+  rm.d_metrics = d_metrics;
+  rm.d_init = stats ? d_init : nullptr;
+  std::vector<RefineLevelStats> rs = level_stats(h, rc, nl, &rm);
+  GKW_REQUIRE(rm.bad == 0, GKW_E_INTERNAL, "partition produced a part id out of range");
+  if (cut_out) *cut_out = rm.cut;
   if (stats) {
     memset(stats, 0, sizeof(*stats));
     stats->n_levels = (i32)lv.size();
@@ -363,11 +361,9 @@ void partition_impl(Handle& h, const DevGraph& g0, i32 k, const gkw_options& opt
       const bool ran = (i + 1 < lv.size()) || balances(nl - 1);
       stats->ms_level[i] = ran ? elapsed_ms(lev[2 * i], lev[2 * i + 1]) : -1.0;
     }
-    stats->init_cut = init_cut;
-    stats->cut = hm[0];
-    i64 mx = 0;
-    for (i32 p = 0; p < k; ++p) mx = std::max(mx, hm[2 + p]);
-    stats->max_part_weight = mx;
+    stats->init_cut = rm.init_cut;
+    stats->cut = rm.cut;
+    stats->max_part_weight = rm.max_pw;
     stats->maxw = maxw;
     stats->ms_coarsen = elapsed_ms(ev[0], ev[1]);
     stats->ms_init = elapsed_ms(ev[1], ev[2]);
@@ -470,11 +466,11 @@ void partition_multi_impl(Handle& h, const DevGraph& g0, i32 nk, const i32* ks, 
     }
     i64* d_metrics = h.hier.alloc_n<i64>(k + 2);
     compute_cut_pw(h, g0, out, k, d_metrics, d_metrics + 2);
-    i64 hm[2] = {0, 0};
-    GKW_CUDA(cudaMemcpyAsync(hm, d_metrics, sizeof(i64) * 2, cudaMemcpyDeviceToHost, h.stream));
-    level_stats(h, rc, nl);   // one sync; error words of the level kernels
-    GKW_REQUIRE(hm[1] == 0, GKW_E_INTERNAL, "partition produced a part id out of range");
-    if (cuts_out) cuts_out[q] = hm[0];
+    RunMetrics rm;
+    rm.d_metrics = d_metrics;
+    level_stats(h, rc, nl, &rm);   // one sync; error words of the level kernels
+    GKW_REQUIRE(rm.bad == 0, GKW_E_INTERNAL, "partition produced a part id out of range");
+    if (cuts_out) cuts_out[q] = rm.cut;
     h.hier.release(mk);
   }
 }

@@ -94,14 +94,16 @@ struct RefineCtx {
   i32* cw = nullptr;     // per candidate list entry: vertex weight
   u32* risk = nullptr;   // per part: 1 if the round's candidates could push it over MAXW
   i32* pnet = nullptr;   // net weight change of each part if every candidate moved
-  RoundState* st = nullptr;
+  RoundState* st = nullptr;    // one per stats slot
   u32* bmark = nullptr;
   i32* btarget = nullptr;
   i32* bgain = nullptr;
   i32* blist = nullptr;
   u32* brem = nullptr;
   u32* epoch = nullptr;   // never reset: marks of earlier rounds stay stale
-  GridBarrier* bar = nullptr;
+  GridBarrier* bar = nullptr;   // one per stats slot
+  std::vector<char> used;       // slots launched on since they were cleared
+  bool pw_clear = false;        // pw is still as cleared
   CountBarrier* cbar = nullptr;   // the refinement rounds' barriers (zeroed before each launch)
   i32* err = nullptr;
   LevelStatsDev* stats = nullptr;
@@ -2599,9 +2601,11 @@ __global__ void __launch_bounds__(kLevelThreads, 1) k_level(LevelArgs a) {
 // ---------------------------------------------------------------------------
 __global__ void k_boundary_pw(i32 n, const i32* __restrict__ xadj, const i32* __restrict__ adjncy,
                               const i32* __restrict__ vwgt, const i32* __restrict__ part,
-                              i32* __restrict__ bnd, u32* __restrict__ pw) {
+                              i32* __restrict__ bnd, u32* __restrict__ pw, i32* __restrict__ updflag,
+                              i32* __restrict__ inP, i32* __restrict__ gain) {
   const i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= n) return;
+  if (updflag) updflag[v] = inP[v] = gain[v] = 0;
   const i32 p = part[v];
   i32 b = 0;
   for (i32 e = xadj[v]; e < xadj[v + 1]; ++e)
@@ -2629,39 +2633,46 @@ static void ctx_common(Handle& h, Pool& P, RefineCtx* c, size_t n) {
   // is a candidate at most once per round, so n entries always suffice
   const bool batched = c->kacc > 0 && c->kacc < c->k;
   c->top = P.alloc_n<u64>(batched ? std::max<size_t>(n, kMaxMoveCap) : kMaxMoveCap);
-  c->pw = P.alloc_n<u32>(c->k);
-  c->pwd = P.alloc_n<u32>(c->k);
-  c->pin = P.alloc_n<u32>(c->k);
   c->msrc = P.alloc_n<i32>(n);
   c->cinfo = P.alloc_n<u64>(n);
   c->cw = P.alloc_n<i32>(n);
-  c->risk = P.alloc_n<u32>(c->k);
-  c->pnet = P.alloc_n<i32>(c->k);
-  c->st = P.alloc_n<RoundState>(1);
-  c->bmark = P.alloc_n<u32>(n);
   c->btarget = P.alloc_n<i32>(n);
   c->bgain = P.alloc_n<i32>(n);
   c->blist = P.alloc_n<i32>(n);
   c->brem = P.alloc_n<u32>(c->k);
-  c->epoch = P.alloc_n<u32>(1);
-  c->bar = P.alloc_n<GridBarrier>(1);
   c->cbar = P.alloc_n<CountBarrier>(1);
-  c->err = P.alloc_n<i32>(1);
-  c->stats = P.alloc_n<LevelStatsDev>(kStatSlots);
+  {   // everything that starts at zero, in one block: one clear a context and none a level
+    const size_t kw = (((size_t)c->k * 4) + 63) & ~(size_t)63;
+    size_t bytes = 0;
+    auto take = [&](size_t b) {
+      const size_t at = bytes;
+      bytes = (bytes + b + 63) & ~(size_t)63;
+      return at;
+    };
+    const size_t o_stats = take(sizeof(LevelStatsDev) * kStatSlots), o_st = take(sizeof(RoundState) * kStatSlots);
+    const size_t o_bar = take(sizeof(GridBarrier) * kStatSlots), o_err = take(4), o_epoch = take(4);
+    const size_t o_k = take(5 * kw), o_bmark = take(sizeof(u32) * n);
+    char* base = reinterpret_cast<char*>(P.alloc(bytes));
+    c->stats = reinterpret_cast<LevelStatsDev*>(base + o_stats);
+    c->st = reinterpret_cast<RoundState*>(base + o_st);
+    c->bar = reinterpret_cast<GridBarrier*>(base + o_bar);
+    c->err = reinterpret_cast<i32*>(base + o_err);
+    c->epoch = reinterpret_cast<u32*>(base + o_epoch);
+    c->pwd = reinterpret_cast<u32*>(base + o_k);   // kept at zero between rounds
+    c->pin = reinterpret_cast<u32*>(base + o_k + kw);
+    c->risk = reinterpret_cast<u32*>(base + o_k + 2 * kw);
+    c->pnet = reinterpret_cast<i32*>(base + o_k + 3 * kw);
+    c->pw = reinterpret_cast<u32*>(base + o_k + 4 * kw);
+    c->bmark = reinterpret_cast<u32*>(base + o_bmark);
+    GKW_CUDA(cudaMemsetAsync(base, 0, bytes, h.stream));
+    c->used.assign(kStatSlots, 0);
+    c->pw_clear = true;
+  }
   if (const char* t = getenv("GKW_TRACE"); t && *t == '1') {
     c->trace = P.alloc_n<u64>((size_t)kStatSlots * kTraceCap);
     c->trace_n = P.alloc_n<i32>(kStatSlots);
     GKW_CUDA(cudaMemsetAsync(c->trace_n, 0, sizeof(i32) * kStatSlots, h.stream));
   }
-  GKW_CUDA(cudaMemsetAsync(c->bmark, 0, sizeof(u32) * n, h.stream));
-  GKW_CUDA(cudaMemsetAsync(c->pwd, 0, sizeof(u32) * c->k, h.stream));   // kept at zero between rounds
-  GKW_CUDA(cudaMemsetAsync(c->pin, 0, sizeof(u32) * c->k, h.stream));
-  GKW_CUDA(cudaMemsetAsync(c->risk, 0, sizeof(u32) * c->k, h.stream));
-  GKW_CUDA(cudaMemsetAsync(c->pnet, 0, sizeof(i32) * c->k, h.stream));
-  GKW_CUDA(cudaMemsetAsync(c->epoch, 0, sizeof(u32), h.stream));
-  GKW_CUDA(cudaMemsetAsync(c->bar, 0, sizeof(GridBarrier), h.stream));
-  GKW_CUDA(cudaMemsetAsync(c->err, 0, sizeof(i32), h.stream));
-  GKW_CUDA(cudaMemsetAsync(c->stats, 0, sizeof(LevelStatsDev) * kStatSlots, h.stream));
   // per-warp part-connection rows: as many warps as fit beside the sort buffer
   const size_t budget = 120 * 1024;
   if (c->kacc <= 0) c->kacc = c->k;
@@ -2729,38 +2740,45 @@ i32* refine_gain(RefineCtx* c) { return c->gain; }
 i32* refine_target(RefineCtx* c) { return c->target; }
 u32* refine_pw(RefineCtx* c) { return c->pw; }
 
+static void clear_part_weights(Handle& h, RefineCtx* c) {
+  if (!c->pw_clear) GKW_CUDA(cudaMemsetAsync(c->pw, 0, sizeof(u32) * c->k, h.stream));
+  c->pw_clear = false;
+}
+
 void refine_init_coarsest(Handle& h, RefineCtx* c, const DevGraph& g, const i32* d_part_in) {
   c->cur = 0;
-  GKW_CUDA(cudaMemsetAsync(c->pw, 0, sizeof(u32) * c->k, h.stream));
+  clear_part_weights(h, c);
   if (g.n == 0) return;
   const u32 nb = ceil_div(g.n, 256);
   if (d_part_in != c->part[0]) {
     launch(k_copy_i32, nb, 256, 0, h.stream, g.n, d_part_in, c->part[0]);
     GKW_CHECK_LAUNCH();
   }
-  launch(k_boundary_pw, nb, 256, 0, h.stream, g.n, g.xadj, g.adjncy, g.vwgt, c->part[0], c->bnd[0], c->pw);
+  launch(k_boundary_pw, nb, 256, 0, h.stream, g.n, g.xadj, g.adjncy, g.vwgt, c->part[0], c->bnd[0], c->pw,
+         c->updflag, c->inP, c->gain);
   GKW_CHECK_LAUNCH();
-  GKW_CUDA(cudaMemsetAsync(c->updflag, 0, sizeof(i32) * g.n, h.stream));
-  GKW_CUDA(cudaMemsetAsync(c->inP, 0, sizeof(i32) * g.n, h.stream));
-  GKW_CUDA(cudaMemsetAsync(c->gain, 0, sizeof(i32) * g.n, h.stream));
 }
 
 void refine_init_union(Handle& h, RefineCtx* c, const DevGraph& cu, const i32* part, i32* bnd_out) {
   c->cur = 0;
-  GKW_CUDA(cudaMemsetAsync(c->pw, 0, sizeof(u32) * c->k, h.stream));
+  clear_part_weights(h, c);
   if (cu.n == 0) return;
   launch(k_boundary_pw, ceil_div(cu.n, 256), 256, 0, h.stream, cu.n, cu.xadj, cu.adjncy, cu.vwgt, part, bnd_out,
-         c->pw);
+         c->pw, (i32*)nullptr, (i32*)nullptr, (i32*)nullptr);
   GKW_CHECK_LAUNCH();
 }
 
 void level_run(Handle& h, RefineCtx* c, const DevGraph& g, const LevelJob& j, i32 slot) {
   GKW_REQUIRE(j.move_cap >= 1 && j.move_cap <= c->cap, GKW_E_INVALID, "move_cap out of range");
   GKW_REQUIRE(slot >= 0 && slot < kStatSlots, GKW_E_INTERNAL, "stats slot out of range");
-  GKW_CUDA(cudaMemsetAsync(c->st, 0, sizeof(RoundState), h.stream));
-  // barrier words start from zero for every launch; an error of an earlier
-  // level stays in c->err, so every later level leaves at its first barrier
-  GKW_CUDA(cudaMemsetAsync(c->bar, 0, sizeof(GridBarrier), h.stream));
+  // round state and barrier words start from zero for every launch; an error
+  // of an earlier level stays in c->err, so every later level leaves at its
+  // first barrier
+  if (c->used[slot]) {
+    GKW_CUDA(cudaMemsetAsync(c->st + slot, 0, sizeof(RoundState), h.stream));
+    GKW_CUDA(cudaMemsetAsync(c->bar + slot, 0, sizeof(GridBarrier), h.stream));
+  }
+  c->used[slot] = 1;
   LevelArgs a;
   memset(&a, 0, sizeof(a));
   a.n = g.n;
@@ -2818,14 +2836,14 @@ void level_run(Handle& h, RefineCtx* c, const DevGraph& g, const LevelJob& j, i3
   a.cw = c->cw;
   a.risk = c->risk;
   a.pnet = c->pnet;
-  a.st = c->st;
+  a.st = c->st + slot;
   a.bmark = c->bmark;
   a.btarget = c->btarget;
   a.bgain = c->bgain;
   a.blist = c->blist;
   a.brem = c->brem;
   a.epoch = c->epoch;
-  a.bar = c->bar;
+  a.bar = c->bar + slot;
   a.cbar = c->cbar;
   a.err = c->err;
   a.stat_slot = c->stats + slot;
@@ -2864,16 +2882,56 @@ void level_run(Handle& h, RefineCtx* c, const DevGraph& g, const LevelJob& j, i3
   c->cur = dst;
 }
 
-std::vector<RefineLevelStats> level_stats(Handle& h, RefineCtx* c, i32 nslots) {
-  GKW_REQUIRE(nslots >= 0 && nslots <= kStatSlots, GKW_E_INTERNAL, "stats slot out of range");
-  std::vector<LevelStatsDev> d((size_t)std::max(nslots, 1));
-  if (nslots) {
-    GKW_CUDA(cudaMemcpyAsync(d.data(), c->stats, sizeof(LevelStatsDev) * nslots, cudaMemcpyDeviceToHost,
-                             h.stream));
+// The end of a run in one read: the level kernels' statistics and error word,
+// the cut, the bad-part flag and the heaviest part (and the initial
+// partition's cut), written straight to the handle's pinned words.
+struct EndReport {
+  i32 err, pad;
+  i64 cut, bad, max_pw, init_cut;
+  LevelStatsDev stats[kStatSlots];
+};
+static_assert(sizeof(EndReport) <= kPinnedWords * sizeof(i64), "pinned words too few");
+
+__global__ void __launch_bounds__(256) k_end_report(const LevelStatsDev* stats, i32 nslots, const i32* err,
+                                                    const i64* metrics, i32 k, const i64* init, EndReport* out) {
+  const i64* src = reinterpret_cast<const i64*>(stats);
+  i64* dst = reinterpret_cast<i64*>(out->stats);
+  static_assert(sizeof(LevelStatsDev) % 8 == 0, "copied by words");
+  for (i32 i = threadIdx.x; i < nslots * (i32)(sizeof(LevelStatsDev) / 8); i += blockDim.x) dst[i] = src[i];
+  __shared__ i64 s_max[8];
+  i64 mx = 0;
+  if (metrics)
+    for (i32 p = threadIdx.x; p < k; p += blockDim.x) mx = max(mx, metrics[2 + p]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = mx;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) mx = max(mx, s_max[w]);
+    out->err = *err;
+    out->cut = metrics ? metrics[0] : 0;
+    out->bad = metrics ? metrics[1] : 0;
+    out->max_pw = mx;
+    out->init_cut = init ? init[0] : 0;
   }
-  GKW_CUDA(cudaMemcpyAsync(h.h_pinned, c->err, sizeof(i32), cudaMemcpyDeviceToHost, h.stream));
+}
+
+std::vector<RefineLevelStats> level_stats(Handle& h, RefineCtx* c, i32 nslots, RunMetrics* metrics) {
+  GKW_REQUIRE(nslots >= 0 && nslots <= kStatSlots, GKW_E_INTERNAL, "stats slot out of range");
+  EndReport* rep = reinterpret_cast<EndReport*>(h.h_pinned);
+  launch(k_end_report, 1, 256, 0, h.stream, (const LevelStatsDev*)c->stats, nslots, (const i32*)c->err,
+         metrics ? metrics->d_metrics : (const i64*)nullptr, c->k, metrics ? metrics->d_init : (const i64*)nullptr,
+         rep);
+  GKW_CHECK_LAUNCH();
   GKW_CUDA(cudaStreamSynchronize(h.stream));
-  const i32 err = *(i32*)h.h_pinned;
+  std::vector<LevelStatsDev> d(rep->stats, rep->stats + nslots);
+  const i32 err = rep->err;
+  if (metrics) {
+    metrics->cut = rep->cut;
+    metrics->bad = rep->bad;
+    metrics->max_pw = rep->max_pw;
+    metrics->init_cut = rep->init_cut;
+  }
   if (err == 1) throw Error{GKW_E_INTERNAL, "level kernel: grid barrier timed out"};
   if (err == 2) throw Error{GKW_E_INTERNAL, "balancing did not terminate"};
   if (err == 3) throw Error{GKW_E_INTERNAL, "refinement did not terminate"};
@@ -3029,9 +3087,9 @@ void launch_cut_pw(cudaStream_t stream, i32 sm_count, const DevGraph& g, const i
   GKW_CHECK_LAUNCH();
 }
 
-void compute_cut_pw(Handle& h, const DevGraph& g, const i32* part, i32 k, i64* d_cut, i64* d_pw) {
+void compute_cut_pw(Handle& h, const DevGraph& g, const i32* part, i32 k, i64* d_cut, i64* d_pw, bool cleared) {
   GKW_REQUIRE(d_pw == d_cut + 2, GKW_E_INTERNAL, "cut accumulators must be contiguous");
-  GKW_CUDA(cudaMemsetAsync(d_cut, 0, sizeof(i64) * (k + 2), h.stream));   // [0] cut, [1] bad-part flag, pw
+  if (!cleared) GKW_CUDA(cudaMemsetAsync(d_cut, 0, sizeof(i64) * (k + 2), h.stream));   // [0] cut, [1] bad-part flag, pw
   launch_cut_pw(h.stream, h.sm_count, g, part, k, d_cut);
 }
 
