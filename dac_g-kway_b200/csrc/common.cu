@@ -172,8 +172,137 @@ __device__ __forceinline__ u64 ld_relaxed_gpu_u64(const unsigned long long* p) {
   return v;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_1pass(const i32* in, i32* out, i64 n, i32* total,
-                                                             ScanState* ss, i32 ntiles) {
+// What a scan's threads load: eight consecutive values each, as 16-byte words
+// where the array allows it.
+//   kScanChunks  the input holds group sizes and the values scanned are the
+//     coarse ids each group takes, ceil(size / cap); a group above the cap also
+//     takes its block of the member list here, from a counter with one atomic
+//     per warp (the blocks' order does not matter, since every group is
+//     ordered within its own block); (size, first id) pairs go out
+//   kScanSums    the input holds 64-bit words, weight << 32 | row length: the
+//     lengths are scanned, and both halves are written out as arrays; `last`
+//     is cleared at the scan's last element
+enum { kScanPlain, kScanChunks, kScanSums };
+struct ScanExtra {
+  i32 cap = 1;
+  i32* goff = nullptr;       // chunks: block of a group above the cap
+  i32* mcounter = nullptr;
+  i32 *weight = nullptr, *length = nullptr, *last = nullptr;   // sums
+};
+
+template <int kMode>
+__device__ __forceinline__ i32 scan_load(const i32* in, i64 b0, i64 n, const ScanExtra& ca, i32 (&v)[kScanItems]) {
+  static_assert(kScanItems == 8, "two 16-byte words");
+  if (kMode == kScanSums) {
+    const ulonglong2* p = reinterpret_cast<const ulonglong2*>(reinterpret_cast<const u64*>(in) + b0);
+    u64 w[kScanItems];
+#pragma unroll
+    for (int i = 0; i < kScanItems; i += 2) {   // (the word array is padded to whole pairs)
+      const ulonglong2 x = b0 + i < n ? p[i / 2] : make_ulonglong2(0, 0);
+      w[i] = x.x;
+      w[i + 1] = b0 + i + 1 < n ? x.y : 0;
+    }
+    i32 sum = 0;
+    i32 wt[kScanItems];
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) {
+      v[i] = (i32)(u32)w[i];
+      wt[i] = (i32)(u32)(w[i] >> 32);
+      sum += v[i];
+    }
+    if (b0 + kScanItems < n) {   // (both arrays are the pool's: aligned)
+      int4* pl = reinterpret_cast<int4*>(ca.length + b0);
+      int4* pw = reinterpret_cast<int4*>(ca.weight + b0);
+      pl[0] = make_int4(v[0], v[1], v[2], v[3]);
+      pl[1] = make_int4(v[4], v[5], v[6], v[7]);
+      pw[0] = make_int4(wt[0], wt[1], wt[2], wt[3]);
+      pw[1] = make_int4(wt[4], wt[5], wt[6], wt[7]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < kScanItems; ++i) {
+        if (b0 + i < n) ca.length[b0 + i] = v[i];
+        if (b0 + i < n - 1) ca.weight[b0 + i] = wt[i];
+        if (b0 + i == n - 1) ca.last[b0 + i] = 0;
+      }
+    }
+    return sum;
+  }
+  if (b0 + kScanItems <= n && (reinterpret_cast<uintptr_t>(in) & 15) == 0) {
+    const int4 x = *reinterpret_cast<const int4*>(in + b0), y = *reinterpret_cast<const int4*>(in + b0 + 4);
+    v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w, v[4] = y.x, v[5] = y.y, v[6] = y.z, v[7] = y.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) v[i] = (b0 + i < n) ? in[b0 + i] : 0;
+  }
+  if (kMode == kScanChunks) {
+    i32 big = 0;
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) big += v[i] > ca.cap ? v[i] : 0;
+    const int lane = threadIdx.x & 31;
+    i32 inc = big;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const i32 y = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += y;
+    }
+    i32 base = 0;
+    if (lane == 31 && inc) base = atomicAdd(ca.mcounter, inc);
+    base = __shfl_sync(0xffffffffu, base, 31) + inc - big;
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) {
+      if (v[i] > ca.cap) {
+        ca.goff[b0 + i] = base;
+        base += v[i];
+        v[i] = (v[i] - 1) / ca.cap + 1;
+      } else {
+        v[i] = v[i] > 0;
+      }
+    }
+  }
+  i32 sum = 0;
+#pragma unroll
+  for (int i = 0; i < kScanItems; ++i) sum += v[i];
+  return sum;
+}
+
+// kScanChunks: `size` holds the group sizes
+template <int kMode>
+__device__ __forceinline__ void scan_store(i32* out, i64 b0, i64 n, i32 run, const i32 (&v)[kScanItems],
+                                           const i32* size) {
+  if constexpr (kMode == kScanChunks) {   // (pairs of records, aligned as `out` is: the pool's)
+    int4* rec = reinterpret_cast<int4*>(out) + b0 / 2;
+#pragma unroll
+    for (int i = 0; i < kScanItems; i += 2) {
+      const i32 a = run, b = run + v[i];
+      run = b + v[i + 1];
+      if (b0 + i + 1 < n) rec[i / 2] = make_int4(size[b0 + i], a, size[b0 + i + 1], b);
+      else if (b0 + i < n) reinterpret_cast<int2*>(out)[b0 + i] = make_int2(size[b0 + i], a);
+    }
+    return;
+  } else {
+    i32 r[kScanItems];
+#pragma unroll
+    for (int i = 0; i < kScanItems; ++i) {
+      r[i] = run;
+      run += v[i];
+    }
+    if (b0 + kScanItems <= n && (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
+      *reinterpret_cast<int4*>(out + b0) = make_int4(r[0], r[1], r[2], r[3]);
+      *reinterpret_cast<int4*>(out + b0 + 4) = make_int4(r[4], r[5], r[6], r[7]);
+    } else {
+#pragma unroll
+      for (int i = 0; i < kScanItems; ++i)
+        if (b0 + i < n) out[b0 + i] = r[i];
+    }
+  }
+}
+
+// d_last: the scan ends with element *d_last (at most n - 1): a level's coarse
+// arrays are sized by its fine vertices, and three of four of their tiles lie
+// beyond n_c.
+template <int kMode>
+__global__ void __launch_bounds__(kScanThreads) k_scan_1pass(const i32* in, i32* out, i64 n, const i32* d_last,
+                                                             i32* total, ScanState* ss, i32 ntiles, ScanExtra ca) {
   __shared__ i32 s_warp[33];
   __shared__ i32 s_tile;
   __shared__ i32 s_excl;
@@ -182,71 +311,67 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_1pass(const i32* in, i32*
     s_tile = (i32)atomicAdd(&ss->ticket, 1u);
     s_epoch = *(volatile u32*)&ss->epoch;   // set by the previous scan, stream-ordered before this one
   }
+  if (d_last) {
+    const i64 last = *d_last;
+    n = last + 1 < n ? last + 1 : n;
+  }
   __syncthreads();
   const i32 tile = s_tile;
   const u64 epoch = s_epoch;
   const i64 b0 = (i64)tile * kScanTile + (i64)threadIdx.x * kScanItems;
-  i32 v[kScanItems];
-  i32 sum = 0;
-#pragma unroll
-  for (int i = 0; i < kScanItems; ++i) {
-    v[i] = (b0 + i < n) ? in[b0 + i] : 0;
-    sum += v[i];
-  }
-  i32 agg;
-  const i32 off = block_exclusive_scan(sum, s_warp, agg);
-  if (threadIdx.x < 32) {
-    // warp 0 looks back 32 predecessors per step: every lane waits for its
-    // predecessor's word, the nearest inclusive prefix ends the walk
-    const int lane = threadIdx.x;
-    unsigned long long* st = (unsigned long long*)ss->tiles;
-    const u64 tag = epoch << 34;
-    i32 excl = 0;
-    if (tile == 0) {
-      if (lane == 0) atomicExch(&st[0], (unsigned long long)(tag | (2ull << 32) | (u32)agg));
-    } else {
-      if (lane == 0) atomicExch(&st[tile], (unsigned long long)(tag | (1ull << 32) | (u32)agg));
-      i64 hi = (i64)tile - 1;
-      const long long t0 = clock64();
-      for (;;) {
-        const i64 j = hi - lane;
-        u32 status = 2, val = 0;   // before tile 0: an empty prefix
-        if (j >= 0) {
-          for (;;) {
-            const u64 w = ld_relaxed_gpu_u64(&st[j]);
-            status = (w >> 34) == epoch ? (u32)((w >> 32) & 3u) : 0u;
-            val = (u32)w;
-            if (status != 0) break;
-            if (clock64() - t0 > kScanSpinCycles) {
-              atomicExch(&ss->err, 1);
-              status = 2;
-              val = 0;
-              break;
+  if ((i64)tile * kScanTile < n) {   // (no tile looks back at one beyond the end)
+    i32 v[kScanItems];
+    const i32 sum = scan_load<kMode>(in, b0, n, ca, v);
+    i32 agg;
+    const i32 off = block_exclusive_scan(sum, s_warp, agg);
+    if (threadIdx.x < 32) {
+      // warp 0 looks back 32 predecessors per step: every lane waits for its
+      // predecessor's word, the nearest inclusive prefix ends the walk
+      const int lane = threadIdx.x;
+      unsigned long long* st = (unsigned long long*)ss->tiles;
+      const u64 tag = epoch << 34;
+      i32 excl = 0;
+      if (tile == 0) {
+        if (lane == 0) atomicExch(&st[0], (unsigned long long)(tag | (2ull << 32) | (u32)agg));
+      } else {
+        if (lane == 0) atomicExch(&st[tile], (unsigned long long)(tag | (1ull << 32) | (u32)agg));
+        i64 hi = (i64)tile - 1;
+        const long long t0 = clock64();
+        for (;;) {
+          const i64 j = hi - lane;
+          u32 status = 2, val = 0;   // before tile 0: an empty prefix
+          if (j >= 0) {
+            for (;;) {
+              const u64 w = ld_relaxed_gpu_u64(&st[j]);
+              status = (w >> 34) == epoch ? (u32)((w >> 32) & 3u) : 0u;
+              val = (u32)w;
+              if (status != 0) break;
+              if (clock64() - t0 > kScanSpinCycles) {
+                atomicExch(&ss->err, 1);
+                status = 2;
+                val = 0;
+                break;
+              }
             }
           }
+          const u32 m2 = __ballot_sync(0xffffffffu, status == 2);
+          const int first2 = m2 ? __ffs(m2) - 1 : 32;   // nearest published prefix
+          i32 add = lane <= first2 ? (i32)val : 0;
+  #pragma unroll
+          for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
+          excl += add;
+          if (m2) break;
+          hi -= 32;
         }
-        const u32 m2 = __ballot_sync(0xffffffffu, status == 2);
-        const int first2 = m2 ? __ffs(m2) - 1 : 32;   // nearest published prefix
-        i32 add = lane <= first2 ? (i32)val : 0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) add += __shfl_xor_sync(0xffffffffu, add, o);
-        excl += add;
-        if (m2) break;
-        hi -= 32;
+        if (lane == 0) atomicExch(&st[tile], (unsigned long long)(tag | (2ull << 32) | (u32)(excl + agg)));
       }
-      if (lane == 0) atomicExch(&st[tile], (unsigned long long)(tag | (2ull << 32) | (u32)(excl + agg)));
+      if (lane == 0) {
+        s_excl = excl;
+        if (tile == (i32)((n - 1) / kScanTile) && total) *total = excl + agg;
+      }
     }
-    if (lane == 0) {
-      s_excl = excl;
-      if (tile == ntiles - 1 && total) *total = excl + agg;
-    }
-  }
-  __syncthreads();
-  i32 run = off + s_excl;
-#pragma unroll
-  for (int i = 0; i < kScanItems; ++i) {
-    if (b0 + i < n) out[b0 + i] = run;
-    run += v[i];
+    __syncthreads();
+    scan_store<kMode>(out, b0, n, off + s_excl, v, in);
   }
   if (threadIdx.x == 0) {
     // the last tile to finish: every other tile has taken its ticket, read
@@ -266,34 +391,32 @@ __global__ void k_set_i32(i32* p, i32 v) { *p = v; }
 // A scan that fits one tile: one CTA, no tickets, status words or look-back
 // (the single-pass scan's bookkeeping is several dependent round trips to L2,
 // most of a small scan's time).
-__global__ void __launch_bounds__(kScanThreads) k_scan_small(const i32* in, i32* out, i32 n, i32* total) {
+template <int kMode>
+__global__ void __launch_bounds__(kScanThreads) k_scan_small(const i32* in, i32* out, i32 n, const i32* d_last,
+                                                             i32* total, ScanExtra ca) {
   __shared__ i32 s_warp[33];
   const i32 b0 = threadIdx.x * kScanItems;
+  if (d_last) {
+    const i32 last = *d_last;
+    n = last < n ? last + 1 : n;
+  }
   i32 v[kScanItems];
-  i32 sum = 0;
-#pragma unroll
-  for (int i = 0; i < kScanItems; ++i) {
-    v[i] = (b0 + i < n) ? in[b0 + i] : 0;
-    sum += v[i];
-  }
+  const i32 sum = scan_load<kMode>(in, b0, n, ca, v);
   i32 agg;
-  i32 run = block_exclusive_scan(sum, s_warp, agg);
-#pragma unroll
-  for (int i = 0; i < kScanItems; ++i) {
-    if (b0 + i < n) out[b0 + i] = run;
-    run += v[i];
-  }
+  const i32 run = block_exclusive_scan(sum, s_warp, agg);
+  scan_store<kMode>(out, b0, n, run, v, in);
   if (threadIdx.x == 0 && total) *total = agg;
 }
 
-void exclusive_scan_i32(Handle& h, const i32* in, i32* out, i64 n, i32* total) {
+template <int kMode>
+static void scan_i32(Handle& h, const i32* in, i32* out, i64 n, i32* total, const i32* d_last, ScanExtra ca) {
   if (n <= 0) {
     if (total) launch(k_set_i32, 1, 1, 0, h.stream, total, 0);
     GKW_CHECK_LAUNCH();
     return;
   }
   if (n <= kScanTile) {
-    launch(k_scan_small, 1, kScanThreads, 0, h.stream, in, out, (i32)n, total);
+    launch(k_scan_small<kMode>, 1, kScanThreads, 0, h.stream, in, out, (i32)n, d_last, total, ca);
     GKW_CHECK_LAUNCH();
     return;
   }
@@ -323,8 +446,29 @@ void exclusive_scan_i32(Handle& h, const i32* in, i32* out, i64 n, i32* total) {
   }
   h.scan_epoch += 1;   // host mirror of the device epoch (wrap guard only)
   ++h.scans_enqueued;
-  launch(k_scan_1pass, nt, kScanThreads, 0, h.stream, in, out, n, total, h.scan, nt);
+  launch(k_scan_1pass<kMode>, nt, kScanThreads, 0, h.stream, in, out, n, d_last, total, h.scan, nt, ca);
   GKW_CHECK_LAUNCH();
+}
+
+void exclusive_scan_i32(Handle& h, const i32* in, i32* out, i64 n, i32* total, const i32* d_last) {
+  scan_i32<kScanPlain>(h, in, out, n, total, d_last, ScanExtra{});
+}
+
+void scan_group_chunks(Handle& h, const i32* gsize, int2* grec, i32* goff, i32* mcounter, i64 n, i32 cap, i32* total) {
+  ScanExtra x;
+  x.cap = cap;
+  x.goff = goff;
+  x.mcounter = mcounter;
+  scan_i32<kScanChunks>(h, gsize, reinterpret_cast<i32*>(grec), n, total, nullptr, x);
+}
+
+void scan_coarse_sums(Handle& h, const u64* sums, i32* ub, i32* rowlen, i32* cvwgt, i32* cnt, i64 n, i32* total,
+                      const i32* d_last) {
+  ScanExtra x;
+  x.weight = cvwgt;
+  x.length = rowlen;
+  x.last = cnt;
+  scan_i32<kScanSums>(h, reinterpret_cast<const i32*>(sums), ub, n, total, d_last, x);
 }
 
 namespace {

@@ -285,7 +285,18 @@ inline void launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, c
 // ---- device primitives (scan.cu) ----
 // Exclusive scan of `in` (n entries) into `out` (n entries); if `total` is not
 // null, the grand total is stored there (device pointer).  `in` may equal `out`.
-void exclusive_scan_i32(Handle& h, const i32* in, i32* out, i64 n, i32* total);
+// d_last (device, may be null): the scan ends with element *d_last, and the
+// rest of `out` is left as it is.
+void exclusive_scan_i32(Handle& h, const i32* in, i32* out, i64 n, i32* total, const i32* d_last = nullptr);
+// Exclusive scan of ceil(gsize / cap); grec: (size, exclusive sum); each group above the cap
+// gets a block of its size from *mcounter (zero before) in goff.
+void scan_group_chunks(Handle& h, const i32* gsize, int2* grec, i32* goff, i32* mcounter, i64 n, i32 cap, i32* total);
+// sums[c] = weight << 32 | row length (16-byte aligned, an even count of
+// words): exclusive scan of the lengths into ub, the halves into rowlen and
+// cvwgt (cvwgt without the last element, the end of the coarse vertices), and
+// zero into cnt's last element.
+void scan_coarse_sums(Handle& h, const u64* sums, i32* ub, i32* rowlen, i32* cvwgt, i32* cnt, i64 n, i32* total,
+                      const i32* d_last);
 
 // ---- coarsening (coarsen.cu) ----
 // maxdeg: the longest row if known (< 0: unknown); rows above the sub-warp
