@@ -1295,32 +1295,33 @@ __global__ void __launch_bounds__(WARPS * 32) k_contract_warp(
 // Heavy rows (longer than the warp tables) by direct accumulation: one CTA per
 // row, a weight per coarse id in shared memory (kDenseIds ids at a time, a
 // window of the id range) and a bit per id that was met, whose order is the
-// row's -- no hashing, no sort.  It takes every heavy row of levels with at
-// most kDenseIds coarse vertices, and on larger ones the rows beyond the
-// shared table of k_contract_cta, window by window (at most kDenseWindows),
-// whose global table and global sort made a circuit graph's few hub rows the
-// last to finish (heavy rows of all levels of a 4M-vertex circuit graph 6.8
-// ms, now 2.7).
+// row's -- no hashing, no sort.  On levels of more than kDenseIds coarse
+// vertices the row's own range of ids is found first, and the windows cover
+// that: a union of many graphs has millions of ids, its rows one graph's few
+// thousand.  Rows that would take more than kDenseWindows windows
+// (kDenseNear, if the shared table of k_contract_cta holds them) are left to
+// that kernel, whose hashing and sorting cost about as much as that many
+// windows (heavy rows of all levels of a 4M-vertex circuit graph 6.8 ms by
+// hashing alone, now 1.8).
 constexpr i32 kDenseThreads = 1024;
 constexpr i32 kDenseIds = 53248;
 constexpr i32 kDenseWindows = 32;
+constexpr i32 kDenseNear = 4;
 constexpr size_t kDenseSmem = (size_t)kDenseIds * 4 + kDenseIds / 8;
 constexpr i32 kCtaCap = 4096;   // k_contract_cta: longest row of its shared table
 
-__device__ __forceinline__ bool dense_row(i32 nc, i32 L) {
-  return nc <= kDenseIds || (L > kCtaCap && (i64)nc <= (i64)kDenseIds * kDenseWindows);
-}
-
+// rest, nrest: the rows left to k_contract_cta
 __global__ void __launch_bounds__(kDenseThreads, 1) k_contract_dense(
     const i32* __restrict__ ncp, const i32* __restrict__ heavy, const i32* __restrict__ nheavy,
     const i32* __restrict__ xadj, const i32* __restrict__ adjncy, const i32* __restrict__ adjwgt,
     const i32* __restrict__ cmap, const i32* __restrict__ memtab, const i32* __restrict__ mcnt, i32 cap,
     const i32* __restrict__ rowlen, const i32* __restrict__ ub, i32* __restrict__ sadj, i32* __restrict__ swgt,
-    i32* __restrict__ cnt) {
+    i32* __restrict__ cnt, i32* __restrict__ rest, i32* __restrict__ nrest) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   u32* acc = reinterpret_cast<u32*>(smem_raw);         // [kDenseIds]
   u32* bits = acc + kDenseIds;                         // [kDenseIds / 32]
   __shared__ i32 s_warp[kDenseThreads / 32];
+  __shared__ i32 s_lo, s_hi;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const i32 nc = *ncp, nh = *nheavy;
   if (nh == 0) return;
@@ -1328,11 +1329,8 @@ __global__ void __launch_bounds__(kDenseThreads, 1) k_contract_dense(
   __syncthreads();
   for (i32 b = blockIdx.x; b < nh; b += gridDim.x) {
     const i32 c = heavy[b];
-    if (!dense_row(nc, rowlen[c])) continue;   // block-uniform
     const i32 nm = mcnt[c], o = ub[c];
-    i32 U = 0;
-    for (i32 w0 = 0; w0 < nc; w0 += kDenseIds) {
-      const u32 wn = (u32)(nc - w0 < kDenseIds ? nc - w0 : kDenseIds);
+    auto entries = [&](auto visit) {         // visit(coarse id, weight) by every thread's entries, none of them c
       for (i32 j0 = 0; j0 < nm; j0 += 4) {   // four member rows together
         i32 beg[4], end[4];
 #pragma unroll
@@ -1354,16 +1352,52 @@ __global__ void __launch_bounds__(kDenseThreads, 1) k_contract_dense(
           more = false;
 #pragma unroll
           for (i32 q = 0; q < 4; ++q) {
-            const u32 id = (u32)(u[q] - w0);
-            if (u[q] >= 0 && u[q] != c && id < wn) {
-              atomicAdd(&acc[id], (u32)w[q]);
-              atomicOr(&bits[id >> 5], 1u << (id & 31));
-            }
+            if (u[q] >= 0 && u[q] != c) visit(u[q], (u32)w[q]);
             beg[q] += kDenseThreads;
             more |= beg[q] < end[q];
           }
         }
       }
+    };
+    i32 lo = 0, hi = nc - 1;
+    if (nc > kDenseIds) {   // block-uniform
+      if (threadIdx.x == 0) {
+        s_lo = INT_MAX;
+        s_hi = -1;
+      }
+      __syncthreads();
+      lo = INT_MAX;
+      hi = -1;
+      entries([&](i32 u, u32) {
+        lo = u < lo ? u : lo;
+        hi = u > hi ? u : hi;
+      });
+      lo = __reduce_min_sync(kFull, lo);
+      hi = __reduce_max_sync(kFull, hi);
+      if (lane == 0) {
+        atomicMin(&s_lo, lo);
+        atomicMax(&s_hi, hi);
+      }
+      __syncthreads();
+      lo = s_lo;
+      hi = s_hi;
+      __syncthreads();
+      if (hi >= 0 && (hi - lo) / kDenseIds >= (rowlen[c] > kCtaCap ? kDenseWindows : kDenseNear)) {   // block-uniform
+        if (threadIdx.x == 0) rest[atomicAdd(nrest, 1)] = c;
+        continue;
+      }
+    }
+    i32 U = 0;
+    for (i64 w1 = lo; w1 <= hi; w1 += kDenseIds) {
+      const i32 w0 = (i32)w1;
+      const u32 wn = (u32)(hi - w0 < kDenseIds - 1 ? hi - w0 + 1 : kDenseIds);
+      entries([&](i32 u, u32 w) {
+        const u32 id = (u32)(u - w0);
+        if (id < wn) {
+          atomicAdd(&acc[id], w);
+          atomicOr(&bits[id >> 5], 1u << (id & 31));
+        }
+      });
       __syncthreads();
       // the met ids in order: kDenseIds / 32 / kDenseThreads words a thread
       constexpr i32 kW = (kDenseIds / 32 + kDenseThreads - 1) / kDenseThreads;
@@ -1415,7 +1449,7 @@ __global__ void __launch_bounds__(kDenseThreads, 1) k_contract_dense(
 // needs and sets the overflow flag; the host grows the arena and runs the
 // contraction again.  Both kinds of row run in one launch.
 __global__ void __launch_bounds__(512) k_contract_cta(
-    const i32* __restrict__ ncp, const i32* __restrict__ heavy, const i32* __restrict__ nheavy, i32 cta_cap,
+    const i32* __restrict__ heavy, const i32* __restrict__ nheavy, i32 cta_cap,
     const i32* __restrict__ xadj, const i32* __restrict__ adjncy, const i32* __restrict__ adjwgt,
     const i32* __restrict__ cmap, const i32* __restrict__ memtab, const i32* __restrict__ mcnt, i32 cap,
     const i32* __restrict__ rowlen, const i32* __restrict__ ub, i32* __restrict__ sadj,
@@ -1423,11 +1457,10 @@ __global__ void __launch_bounds__(512) k_contract_cta(
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ i32 s_count;
   __shared__ u64 s_off;
-  const i32 nc = *ncp, nh = *nheavy;
+  const i32 nh = *nheavy;
   for (i32 b = blockIdx.x; b < nh; b += gridDim.x) {
     const i32 c = heavy[b];
     const i32 L = rowlen[c];
-    if (dense_row(nc, L)) continue;   // k_contract_dense takes it (block-uniform)
     const bool global_table = L > cta_cap;   // block-uniform
     u32 hsz = 64;
     while (hsz < 2u * (u32)L) hsz <<= 1;
@@ -1597,7 +1630,7 @@ void ensure_arena(Handle& h, u64 words) {
 // The tables that the row kernels share.
 struct ContractTables {
   i32 *rowlen, *ub, *mcnt, *memtab, *cnt, *heavy, *mid;
-  i32* misc;   // [0] heavy rows, [1] ub total, [2] rows listed by the short kernel
+  i32* misc;   // [0] heavy rows, [1] ub total, [2..4] rows listed by the short, the 512 and the dense kernel
   i32 *sadj, *swgt;
   size_t nz;
 };
@@ -1768,7 +1801,7 @@ static void contract_rows(Handle& h, const DevGraph& g, const ContractTables& t,
     rows = misc + 2;
     list = mid;
   }
-  auto warps = [&](auto w, auto k) {
+  auto warps = [&](auto w, auto k, i32* over, i32* nover) {   // rows beyond W entries go to `over`
     constexpr int W = decltype(w)::value, WARPS = 8;
     typedef decltype(k) K;
     const size_t sm = sizeof(WarpTable<W>) * WARPS;
@@ -1776,27 +1809,46 @@ static void contract_rows(Handle& h, const DevGraph& g, const ContractTables& t,
     if (!h.capturing)
       GKW_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     launch(kern, gridw, WARPS * 32, sm, h.stream, rows, list, g.xadj, g.adjncy, g.adjwgt, cmap, memtab, mcnt, cap,
-           rowlen, ub, sadj, swgt, cnt, heavy, misc);
+           rowlen, ub, sadj, swgt, cnt, over, nover);
   };
-  if (wide_ids) warps(std::integral_constant<int, 128>(), u64());
-  else if (expL <= 100) warps(std::integral_constant<int, 128>(), u32());   // (W below)
-  else if (expL <= 400) warps(std::integral_constant<int, 256>(), u32());
-  else warps(std::integral_constant<int, 512>(), u32());
+  if (wide_ids) warps(std::integral_constant<int, 128>(), u64(), heavy, misc);
+  else if (expL <= 100) warps(std::integral_constant<int, 128>(), u32(), heavy, misc);   // (W below)
+  else if (expL <= 400) warps(std::integral_constant<int, 256>(), u32(), heavy, misc);
+  else warps(std::integral_constant<int, 512>(), u32(), heavy, misc);
   GKW_CHECK_LAUNCH();
+  // Where a row can outgrow the smaller tables, the rows that did go through
+  // the 512 one: a level whose mean hides rows of a few hundred entries (a
+  // union of 256 circuits and meshes: 120k of them) left those to one CTA each
+  // (5.3 ms on its first level, now 0.84).  Smaller levels have too few such
+  // rows: a warp takes longer over one than a CTA (a 30k-vertex circuit's
+  // coarsening 0.56 ms with a CTA each, 0.81 with warps).
+  constexpr i32 kMid512 = 100000;
+  i32 *over = heavy, *nover = misc, *free_list = mid;
+  i32 W = wide_ids || expL <= 100 ? 128 : expL <= 400 ? 256 : 512;
+  auto can_outgrow = [&] { return g.maxdeg < 0 || g.maxdeg * (i64)cap > W || cap > 32; };
+  if (W < 512 && !wide_ids && n > kMid512 && can_outgrow()) {
+    rows = misc;
+    list = heavy;
+    warps(std::integral_constant<int, 512>(), u32(), mid, misc + 3);
+    GKW_CHECK_LAUNCH();
+    W = 512;
+    over = mid;
+    nover = misc + 3;
+    free_list = heavy;
+  }
   // heavy rows: only where a row can outgrow the warp tables.  A shared-memory
   // table up to kCtaCap entries, the arena beyond (2*kCtaCap table slots, a
   // power of two, + kCtaCap sorted outputs: 96 KB)
-  const i32 W = wide_ids || expL <= 100 ? 128 : expL <= 400 ? 256 : 512;
-  if (g.maxdeg < 0 || g.maxdeg * (i64)cap > W || cap > 32) {
+  if (can_outgrow()) {
     const size_t csm = (size_t)kCtaCap * 2 * 4 * 2 + (size_t)kCtaCap * 8;
     if (!h.capturing) {
       GKW_CUDA(cudaFuncSetAttribute(k_contract_dense, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem));
       GKW_CUDA(cudaFuncSetAttribute(k_contract_cta, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
     }
-    launch(k_contract_dense, (u32)h.sm_count, kDenseThreads, kDenseSmem, h.stream, d_nc, heavy, misc, g.xadj,
-           g.adjncy, g.adjwgt, cmap, memtab, mcnt, cap, rowlen, ub, sadj, swgt, cnt);
+    launch(k_contract_dense, (u32)h.sm_count, kDenseThreads, kDenseSmem, h.stream, d_nc, over, nover, g.xadj,
+           g.adjncy, g.adjwgt, cmap, memtab, mcnt, cap, rowlen, ub, sadj, swgt, cnt, free_list, misc + 4);
     if (nc_ub > kDenseIds)
-      launch(k_contract_cta, (u32)h.sm_count * 2, 512, csm, h.stream, d_nc, heavy, misc, kCtaCap, g.xadj, g.adjncy,
+      launch(k_contract_cta, (u32)h.sm_count * 2, 512, csm, h.stream, (const i32*)free_list, (const i32*)(misc + 4), kCtaCap, g.xadj, g.adjncy,
              g.adjwgt, cmap, memtab, mcnt, cap, rowlen, ub, sadj, swgt, cnt, h.arena, words, h.arena_words);
     GKW_CHECK_LAUNCH();
   }
