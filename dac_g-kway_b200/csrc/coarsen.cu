@@ -155,6 +155,9 @@ __global__ void __launch_bounds__(kMatchLongThreads) k_match_long(const i32* __r
   }
 }
 
+// Lanes per vertex by mean degree; defaults 2, 8, 16, 32.  Up to 6.5 entries a
+// row two lanes do: a 12M road graph's match 397 us with four, now 278, a
+// million-vertex mesh's 53, now 49.
 i32 match_bucket(const DevGraph& g) {
   const double avg = g.n ? (double)g.m / g.n : 0.0;
   return avg <= 6.5 ? 0 : avg <= 14 ? 1 : avg <= 28 ? 2 : 3;
