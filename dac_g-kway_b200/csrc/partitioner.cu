@@ -19,9 +19,13 @@ namespace gkw {
 // in range and not the vertex itself, weights >= 0.  Also sums vertex weights.
 // flags[0] bit0 bad xadj, bit1 bad id, bit2 self loop, bit3 negative weight.
 // ---------------------------------------------------------------------------
-// flags[1] receives the longest row.  Rows are checked by G lanes each (G
-// from the average row length); rows longer than kValidateLong are left to
-// k_validate_long, one CTA each, so that a hub row does not hold a lane for
+// flags[1] receives the longest row.  A warp checks R consecutive rows, whose
+// entries are one range, as a flat list four loads a lane together: only an
+// entry that names one of the warp's own rows needs to know its row.  Lanes
+// per row left the loads one at a time (a million-vertex mesh 38 us, now
+// 21; a 12M road graph 344, now 129).  R falls with the mean row, so that a
+// warp has about a thousand entries.  Rows longer than kValidateLong are left
+// to k_validate_long, one CTA each, so that a hub row does not hold a warp for
 // thousands of loads.
 constexpr i32 kValidateLong = 512;
 
@@ -37,31 +41,54 @@ __device__ __forceinline__ i32 validate_entries(i32 v, i32 n, i32 b, i32 e, i32 
   return f;
 }
 
-template <int G>
-__global__ void k_validate(i32 n, i64 m, const i32* __restrict__ xadj, const i32* __restrict__ adjncy,
-                           const i32* __restrict__ adjwgt, const i32* __restrict__ vwgt,
-                           i32* __restrict__ flags, unsigned long long* __restrict__ wsum, i32* __restrict__ longlist,
-                           i32* __restrict__ longcnt) {
-  const i64 t = (i64)blockIdx.x * blockDim.x + threadIdx.x;
-  const i64 v = t / G;
-  const int sub = threadIdx.x & (G - 1);
-  i32 f = 0, deg = 0;
+__global__ void __launch_bounds__(256) k_validate(i32 n, i64 m, i32 R, const i32* __restrict__ xadj,
+                                                  const i32* __restrict__ adjncy, const i32* __restrict__ adjwgt,
+                                                  const i32* __restrict__ vwgt, i32* __restrict__ flags,
+                                                  unsigned long long* __restrict__ wsum, i32* __restrict__ longlist,
+                                                  i32* __restrict__ longcnt) {
+  const int lane0 = threadIdx.x & 31;
+  const i64 v0 = (((i64)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * R;
+  const i64 v = v0 + lane0;
+  i32 f = 0, deg = 0, b = 0, e = 0;
   u64 w = 0;
-  if (v < n) {
-    const i32 b = xadj[v], e = xadj[v + 1];
+  const bool in = lane0 < R && v < n;
+  if (in) {
+    b = xadj[v];
+    e = xadj[v + 1];
     if (e < b || b < 0 || (i64)e > m) f |= 1;
     if (v == 0 && b != 0) f |= 1;
     if (v == n - 1 && (i64)e != m) f |= 1;
-    if (sub == 0) {
-      if (vwgt[v] < 0) f |= 8;
-      w = (u32)vwgt[v];
-    }
-    if (!(f & 1)) {
-      deg = e - b;
-      if (deg > kValidateLong) {
-        if (sub == 0) longlist[atomicAdd(longcnt, 1)] = (i32)v;
-      } else {
-        f |= validate_entries((i32)v, n, b, e, sub, G, adjncy, adjwgt);
+    if (vwgt[v] < 0) f |= 8;
+    w = (u32)vwgt[v];
+    if (!(f & 1)) deg = e - b;
+  }
+  if (v0 < n && !__any_sync(0xffffffffu, f & 1)) {   // (a bad xadj is reported whatever the entries hold)
+    const bool isl = deg > kValidateLong;
+    if (isl) longlist[atomicAdd(longcnt, 1)] = (i32)v;
+    if (!__any_sync(0xffffffffu, isl)) {
+      const i32 rows = (i32)(n - v0 < R ? n - v0 : R);
+      const i32 end = __shfl_sync(0xffffffffu, e, rows - 1);
+      constexpr int U = 4;
+      for (i32 j0 = __shfl_sync(0xffffffffu, b, 0) + lane0; j0 < end; j0 += 32 * U) {
+        i32 u[U], wt[U];
+#pragma unroll
+        for (int x = 0; x < U; ++x) {
+          u[x] = j0 + 32 * x < end ? adjncy[j0 + 32 * x] : 0;
+          wt[x] = j0 + 32 * x < end ? adjwgt[j0 + 32 * x] : 0;
+        }
+#pragma unroll
+        for (int x = 0; x < U; ++x) {
+          const i32 j = j0 + 32 * x;
+          if (wt[x] < 0) f |= 8;
+          if (u[x] < 0 || u[x] >= n) f |= 2;
+          else if ((u64)((i64)u[x] - v0) < (u64)rows && j < end && j >= xadj[u[x]] && j < xadj[u[x] + 1]) f |= 4;
+        }
+      }
+    } else {   // the other rows by the warp, one after the other
+      for (u32 todo = __ballot_sync(0xffffffffu, in && !isl); todo; todo &= todo - 1) {
+        const int q = __ffs(todo) - 1;
+        const i32 bq = __shfl_sync(0xffffffffu, b, q), eq = __shfl_sync(0xffffffffu, e, q);
+        f |= validate_entries((i32)(v0 + q), n, bq, eq, lane0, 32, adjncy, adjwgt);
       }
     }
   }
@@ -131,13 +158,10 @@ i64 validate(Handle& h, const DevGraph& g, i64* maxdeg) {
   GKW_CUDA(cudaMemsetAsync(flags, 0, sizeof(i32) * 6, h.stream));
   if (g.n > 0) {
     const double avg = (double)g.m / g.n;
-    auto go = [&](auto kern, int G) {
-      launch(kern, ceil_div((u64)g.n * G, 256), 256, 0, h.stream, g.n, g.m, g.xadj, g.adjncy, g.adjwgt, g.vwgt,
-             flags, ws, longlist, flags + 4);
-    };
-    if (avg <= 6.5) go(k_validate<4>, 4);
-    else if (avg <= 14) go(k_validate<8>, 8);
-    else go(k_validate<16>, 16);
+    i32 R = 32;
+    while (R > 1 && avg * R > 1024) R >>= 1;
+    launch(k_validate, ceil_div((u64)ceil_div((u64)g.n, (u64)R) * 32, 256), 256, 0, h.stream, g.n, g.m, R, g.xadj,
+           g.adjncy, g.adjwgt, g.vwgt, flags, ws, longlist, flags + 4);
     launch(k_validate_long, (u32)h.sm_count * 2, 256, 0, h.stream, g.n, g.xadj, g.adjncy, g.adjwgt, flags,
            (const i32*)longlist, (const i32*)(flags + 4));
     GKW_CHECK_LAUNCH();
