@@ -139,9 +139,23 @@ __device__ __forceinline__ i64 block_sum_i64(i64 x, i64* s_red) {
   __syncthreads();
   if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = x;
   __syncthreads();
-  i64 r = 0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) r += s_red[w];
-  return r;
+  const int lane = threadIdx.x & 31;
+  return warp_sum_i64(lane < (int)(blockDim.x >> 5) ? s_red[lane] : 0);
+}
+
+// Two sums behind one pair of barriers (s_red: two words a warp).
+__device__ __forceinline__ void block_sum2_i64(i64& x, i64& y, i64* s_red) {
+  x = warp_sum_i64(x);
+  y = warp_sum_i64(y);
+  const int lane = threadIdx.x & 31, nw = (int)(blockDim.x >> 5);
+  __syncthreads();
+  if (lane == 0) {
+    s_red[threadIdx.x >> 5] = x;
+    s_red[nw + (threadIdx.x >> 5)] = y;
+  }
+  __syncthreads();
+  x = warp_sum_i64(lane < nw ? s_red[lane] : 0);
+  y = warp_sum_i64(lane < nw ? s_red[nw + lane] : 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -593,6 +607,15 @@ __device__ __forceinline__ i64 grow_packed(const Packing K, u32* V, u32* B1, u32
   return wR;
 }
 
+// The sum of the counts of the warps before this one, and of all nw <= 32
+// (whole warps; two warp reductions instead of a loop of dependent adds).
+__device__ __forceinline__ i32 warps_before(const i32* s_count, int nw, i32& total) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const i32 x = lane < nw ? s_count[lane] : 0;
+  total = __reduce_add_sync(kFull32, x);
+  return __reduce_add_sync(kFull32, lane < wid ? x : 0);
+}
+
 // Stable bisection of one sub-problem by the whole CTA: the members with
 // side(i) go to [p0, pm), the others to [pm, p1), both in id order.
 template <class Side>
@@ -611,12 +634,8 @@ __device__ void split_members(const GggpArgs& a, const SplitParams& P, i32 s, i3
     const u32 bal = __ballot_sync(kFull32, left);
     if (lane == 0) s_scan[wid] = __popc(bal);
     __syncthreads();
-    i32 before = 0, tot = 0;
-    for (int w = 0; w < nw; ++w) {
-      const i32 x = s_scan[w];
-      before += w < wid ? x : 0;
-      tot += x;
-    }
+    i32 tot;
+    const i32 before = warps_before(s_scan, nw, tot);
     if (in) {
       const i32 rankL = doneL + before + __popc(bal & ((1u << lane) - 1));
       const i32 at = left ? o + rankL : o + nL + (i - rankL);
@@ -674,6 +693,10 @@ __device__ __forceinline__ u64 entry_hash(i32 i, i32 j, i32 w) {
 //   state           per trial: words V, B1 (packed path); first the rows'
 //                   counts by member while the rows are built
 // A sub-problem that does not fit goes to the large list.
+// Growth is 700 cycles a pick; beside it a depth costs about 15k cycles of
+// short passes with a barrier each.  Their sums over the warps' counts by two
+// warp reductions took 2048 vertices, k = 8 (three depths) from 382 to 374 us
+// in all, a million-vertex mesh's six from 239 to 229 us.
 // ---------------------------------------------------------------------------
 constexpr int kSmallThreads = 512;
 constexpr i32 kSmallMax = 4096;            // members
@@ -689,7 +712,7 @@ __host__ __device__ __forceinline__ size_t small_bytes(i64 s, i64 L, i32 trials)
 __global__ void __launch_bounds__(kSmallThreads) k_gggp_small(GggpArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ i32 s_scan[kSmallThreads / 32];
-  __shared__ i64 s_red[kSmallThreads / 32];
+  __shared__ i64 s_red[2 * (kSmallThreads / 32)];
   __shared__ i64 s_cut[kInitTrials], s_dev[kInitTrials];
   __shared__ i32 s_inert[kInitTrials];
   __shared__ i32 s_bad, s_carry, s_maxd;
@@ -721,7 +744,8 @@ __global__ void __launch_bounds__(kSmallThreads) k_gggp_small(GggpArgs a) {
     lsum += a.xadj[v + 1] - a.xadj[v];
     wsum += (u32)a.vwgt[v];
   }
-  const i64 L = block_sum_i64(lsum, s_red);
+  block_sum2_i64(lsum, wsum, s_red);
+  const i64 L = lsum, WS = wsum;
   if (s > kSmallMax || small_bytes(s, L, a.trials) > a.smem) {
     if (threadIdx.x == 0) {
       a.biglist[atomicAdd(a.bigcount + a.depth, 1)] = make_int2(p0, p1);
@@ -729,7 +753,6 @@ __global__ void __launch_bounds__(kSmallThreads) k_gggp_small(GggpArgs a) {
     }
     return;
   }
-  const i64 WS = block_sum_i64(wsum, s_red);
   const SplitParams P = split_params(a, p0, p1, WS);
   int4* hdr = reinterpret_cast<int4*>(smem_raw);
   int2* edge = reinterpret_cast<int2*>(hdr + s);
@@ -759,12 +782,8 @@ __global__ void __launch_bounds__(kSmallThreads) k_gggp_small(GggpArgs a) {
     }
     if (lane == 31) s_scan[wid] = inc;
     __syncthreads();
-    i32 before = s_carry, tot = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-      const i32 x = s_scan[w];
-      before += w < wid ? x : 0;
-      tot += x;
-    }
+    i32 tot;
+    const i32 before = s_carry + warps_before(s_scan, kSmallThreads / 32, tot);
     if (i < s) tmp[i] = make_int4(before + inc - len, len, b, 0);
     __syncthreads();
     if (threadIdx.x == 0) s_carry += tot;
@@ -833,12 +852,8 @@ __global__ void __launch_bounds__(kSmallThreads) k_gggp_small(GggpArgs a) {
     const u32 bal = __ballot_sync(kFull32, active);
     if (lane == 0) s_scan[wid] = __popc(bal);
     __syncthreads();
-    i32 before = doneA, tot = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-      const i32 x = s_scan[w];
-      before += w < wid ? x : 0;
-      tot += x;
-    }
+    i32 tot;
+    const i32 before = doneA + warps_before(s_scan, kSmallThreads / 32, tot);
     if (in) {
       const i32 ra = before + __popc(bal & ((1u << lane) - 1));
       const i32 slot = active ? ra : na + (i - ra);
