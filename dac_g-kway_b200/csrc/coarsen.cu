@@ -1910,8 +1910,8 @@ CoopState read_coop(Handle& h, bool reported) {
 // Fused coarsening step: one persistent launch per level runs every phase of
 // the step above -- heavy-edge candidates, union-find rounds, group sizes and
 // coarse ids, group orders, member lists, contraction, coarse xadj and row
-// compaction -- with grid barriers between the phases instead of about twenty
-// kernel launches and ten memsets.  The phase bodies apply the same rules to
+// compaction -- with grid barriers between the phases instead of a dozen
+// launches and more.  The phase bodies apply the same rules to
 // the same keys as the per-phase kernels, so the level is identical; the
 // scans are grid-wide (each CTA scans a contiguous range after a barrier
 // publishes the CTA sums).  Data written by other CTAs in the launch is read
@@ -2799,8 +2799,9 @@ static std::string level_key(const Handle& h, const DevGraph& g, i32 cap, const 
   return std::string("level", 5) + std::string(reinterpret_cast<const char*>(&k), sizeof(k));
 }
 
-// One coarsening step.  Its launch sequence (about twenty kernels and ten
-// memsets, all sized by the level's n and m) runs through the handle's graph
+// One coarsening step.  Its launch sequence (six kernels on a small level,
+// about fifteen and two clears on a large one, all sized by the level's n and
+// m) runs through the handle's graph
 // cache: repeated partitions of the same graph replay it as one CUDA graph.
 // One host sync per level reads the coarse sizes.
 void coarsen_level(Handle& h, const DevGraph& g, i32 cap, CoarsenOut& out) {
