@@ -1421,13 +1421,17 @@ __global__ void __launch_bounds__(kBigThreads, 1) k_gggp_big(GggpArgs a) {
 }
 
 // M = pos = identity, every vertex in its graph's first part, the root
-// sub-problems' places, and the counters of all depths.
-__global__ void k_gggp_init(GggpArgs a, i32 depths, i32 maxbig, const i32* __restrict__ gid,
+// sub-problems' places, and the counters of all depths.  `other`: M's second
+// buffer.  A depth writes only the places of the members it splits, and
+// k_gggp_rows reads every place: a graph of one part (batched) is never split,
+// so its places must name its own vertices in both buffers from the start.
+__global__ void k_gggp_init(GggpArgs a, i32* other, i32 depths, i32 maxbig, const i32* __restrict__ gid,
                             const i32* __restrict__ gpbase, const i32* __restrict__ part_v0,
                             const i32* __restrict__ part_v1) {
   const i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x;
   if (v < a.n) {
     a.mnext[v] = (i32)v;
+    if (maxbig > 0) other[v] = (i32)v;
     a.pos[v] = (i32)v;
     a.part[v] = gid ? gpbase[gid[v]] : 0;
   }
@@ -1560,7 +1564,7 @@ static void device_init_partition_body(Handle& h, const DevGraph& g, i32 k, doub
       a.g_V = h.scratch.alloc_n<u32>((size_t)kInitTrials * a.v_stride);
   }
   a.mnext = ml[0];
-  launch(k_gggp_init, ceil_div((u64)std::max({n, k, maxbig, depth}), 256), 256, 0, h.stream, a, depth, maxbig,
+  launch(k_gggp_init, ceil_div((u64)std::max({n, k, maxbig, depth}), 256), 256, 0, h.stream, a, ml[1], depth, maxbig,
          batch ? batch->gid : (const i32*)nullptr, batch ? batch->gpbase : (const i32*)nullptr,
          batch ? batch->part_v0 : (const i32*)nullptr, batch ? batch->part_v1 : (const i32*)nullptr);
   GKW_CHECK_LAUNCH();
