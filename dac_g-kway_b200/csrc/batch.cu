@@ -92,13 +92,13 @@ __device__ __forceinline__ void warp_rows(i32 n, i64 v, const i32* __restrict__ 
   }
   const bool isl = e - b > kRowLong;
   if (!isl)
-    for (i32 x = b + sub; x < e; x += kRowLanes) visit((i32)v, x);
+    for (u32 x = (u32)b + sub; x < (u32)e; x += kRowLanes) visit((i32)v, (i32)x);
   for (u32 todo = __ballot_sync(0xffffffffu, isl && sub == 0); todo; todo &= todo - 1) {
     const int src = __ffs(todo) - 1;
     const i32 vl = __shfl_sync(0xffffffffu, (i32)v, src);
     const i32 bl = __shfl_sync(0xffffffffu, b, src), el = __shfl_sync(0xffffffffu, e, src);
 #pragma unroll 4
-    for (i32 x = bl + lane; x < el; x += 32) visit(vl, x);
+    for (u32 x = (u32)bl + lane; x < (u32)el; x += 32) visit(vl, (i32)x);
   }
 }
 

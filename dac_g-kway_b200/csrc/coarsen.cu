@@ -61,12 +61,12 @@ __global__ void __launch_bounds__(256) k_match(i32 n, const i32* __restrict__ xa
     if (skip) {
       if (sub == 0) longlist[atomicAdd(longcnt, 1)] = v;
     } else {
-      for (i32 e = beg + sub; e < end; e += G) {
+      for (u32 e = (u32)beg + sub; e < (u32)end; e += G) {
         const u32 w = (u32)__ldg(adjwgt + e);
         if (w == 0 || w < bw) continue;
         const i32 u = __ldg(adjncy + e);
         const u32 d = (u32)(__ldg(xadj + u + 1) - __ldg(xadj + u));
-        if (w > bw || d < bd) { bw = w; bd = d; bpos = e; bu = u; }
+        if (w > bw || d < bd) { bw = w; bd = d; bpos = (i32)e; bu = u; }
       }
     }
   }
@@ -124,10 +124,10 @@ __global__ void __launch_bounds__(kMatchLongThreads) k_match_long(const i32* __r
         visit((u32)w4.z, u4.z, 4 * c + 2);
         visit((u32)w4.w, u4.w, 4 * c + 3);
       }
-      for (i32 e = (tail > body ? tail : body) + threadIdx.x; e < end; e += blockDim.x)
-        visit((u32)adjwgt[e], adjncy[e], e);
+      for (u32 e = (u32)(tail > body ? tail : body) + threadIdx.x; e < (u32)end; e += blockDim.x)
+        visit((u32)adjwgt[e], adjncy[e], (i32)e);
     } else {
-      for (i32 e = beg + threadIdx.x; e < end; e += blockDim.x) visit((u32)adjwgt[e], adjncy[e], e);
+      for (u32 e = (u32)beg + threadIdx.x; e < (u32)end; e += blockDim.x) visit((u32)adjwgt[e], adjncy[e], (i32)e);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -1335,12 +1335,12 @@ __global__ void __launch_bounds__(kDenseThreads, 1) k_contract_dense(
     const i32 nm = mcnt[c], o = ub[c];
     auto entries = [&](auto visit) {         // visit(coarse id, weight) by every thread's entries, none of them c
       for (i32 j0 = 0; j0 < nm; j0 += 4) {   // four member rows together
-        i32 beg[4], end[4];
+        u32 beg[4], end[4];
 #pragma unroll
         for (i32 q = 0; q < 4; ++q) {
           const i32 v = j0 + q < nm ? memtab[c * (i64)cap + j0 + q] : -1;
-          beg[q] = v >= 0 ? xadj[v] + (i32)threadIdx.x : 0;
-          end[q] = v >= 0 ? xadj[v + 1] : 0;
+          beg[q] = v >= 0 ? (u32)xadj[v] + threadIdx.x : 0;
+          end[q] = v >= 0 ? (u32)xadj[v + 1] : 0;
         }
         bool more = true;
         while (more) {
@@ -1356,7 +1356,7 @@ __global__ void __launch_bounds__(kDenseThreads, 1) k_contract_dense(
 #pragma unroll
           for (i32 q = 0; q < 4; ++q) {
             if (u[q] >= 0 && u[q] != c) visit(u[q], (u32)w[q]);
-            beg[q] += kDenseThreads;
+            if (beg[q] < end[q]) beg[q] += kDenseThreads;   // (a short row's place stays while a longer one goes on)
             more |= beg[q] < end[q];
           }
         }
@@ -1500,7 +1500,7 @@ __global__ void __launch_bounds__(512) k_contract_cta(
     for (i32 j = 0; j < nm; ++j) {
       const i32 v = memtab[c * (i64)cap + j];
       const i32 beg = xadj[v], end = xadj[v + 1];
-      for (i32 e = beg + threadIdx.x; e < end; e += blockDim.x) {
+      for (u32 e = (u32)beg + threadIdx.x; e < (u32)end; e += blockDim.x) {
         const u32 key = (u32)cmap[adjncy[e]];
         if (key != (u32)c) table_add(keys, vals, hsz, key, (u32)adjwgt[e]);
       }
@@ -2002,12 +2002,12 @@ __device__ void fz_match(const FusedArgs& a) {
       if (skip) {
         if (sub == 0) a.longlist[atomicAdd(a.misc + kFzLong, 1)] = v;
       } else {
-        for (i32 e = beg + sub; e < end; e += G) {
+        for (u32 e = (u32)beg + sub; e < (u32)end; e += G) {
           const u32 w = (u32)__ldg(a.adjwgt + e);
           if (w == 0 || w < bw) continue;
           const i32 u = __ldg(a.adjncy + e);
           const u32 d = (u32)(__ldg(a.xadj + u + 1) - __ldg(a.xadj + u));
-          if (w > bw || d < bd) { bw = w; bd = d; bpos = e; bu = u; }
+          if (w > bw || d < bd) { bw = w; bd = d; bpos = (i32)e; bu = u; }
         }
       }
     }
@@ -2054,10 +2054,10 @@ __device__ void fz_match_long(const FusedArgs& a) {
         visit((u32)w4.z, u4.z, 4 * c + 2);
         visit((u32)w4.w, u4.w, 4 * c + 3);
       }
-      for (i32 e = (tail > body ? tail : body) + threadIdx.x; e < end; e += blockDim.x)
-        visit((u32)a.adjwgt[e], a.adjncy[e], e);
+      for (u32 e = (u32)(tail > body ? tail : body) + threadIdx.x; e < (u32)end; e += blockDim.x)
+        visit((u32)a.adjwgt[e], a.adjncy[e], (i32)e);
     } else {
-      for (i32 e = beg + threadIdx.x; e < end; e += blockDim.x) visit((u32)a.adjwgt[e], a.adjncy[e], e);
+      for (u32 e = (u32)beg + threadIdx.x; e < (u32)end; e += blockDim.x) visit((u32)a.adjwgt[e], a.adjncy[e], (i32)e);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -2577,7 +2577,7 @@ __global__ void __launch_bounds__(kFusedThreads, 2) k_coarsen_fused(FusedArgs a)
       for (i32 j = 0; j < nm; ++j) {
         const i32 v = ldcg(a.memtab + c * (i64)cap + j);
         const i32 beg = a.xadj[v], end = a.xadj[v + 1];
-        for (i32 e = beg + threadIdx.x; e < end; e += blockDim.x) {
+        for (u32 e = (u32)beg + threadIdx.x; e < (u32)end; e += blockDim.x) {
           const u32 key = (u32)ldcg(a.cmap + a.adjncy[e]);
           if (key != (u32)c) table_add(tk, tv, hsz, key, (u32)a.adjwgt[e]);
         }

@@ -5,6 +5,12 @@
 
 namespace gkw {
 
+// Walks over CSR rows.  A graph has up to 2^31 - 1 entries, so the next place
+// of a walk can pass 2^31 at the end of the last rows.  Held as i32 it would
+// wrap below the row's end and read in front of the arrays: a walk holds it as
+// u32, or where several loads share it as an i64 beside the count of entries
+// left, or counts from the row's start.
+
 // Grid barrier for a cooperative launch, on one 32-bit word.  Each CTA adds
 // to the word with release semantics: CTA 0 adds 2^31 - (gridDim - 1), the
 // others add 1, so the top bit flips exactly when the last CTA arrives and

@@ -1032,13 +1032,13 @@ __global__ void __launch_bounds__(256) k_gggp_rows(GggpArgs a) {
     u64 hash = 0;
     bool bad = false;
     constexpr i32 kU = 4;   // entries per lane whose loads are issued together
-    for (i32 e0 = b; e0 < e1; e0 += 32 * kU) {
+    i64 at = (i64)b + lane;
+    for (i32 left = e1 - b; left > 0; left -= 32 * kU, at += 32 * kU) {   // (warp-uniform)
       i32 u[kU], w[kU], lu[kU];
 #pragma unroll
       for (i32 x = 0; x < kU; ++x) {
-        const i32 e = e0 + 32 * x + lane;
-        u[x] = e < e1 ? a.adjncy[e] : -1;
-        w[x] = e < e1 ? a.adjwgt[e] : 0;
+        u[x] = left - lane > 32 * x ? a.adjncy[at + 32 * x] : -1;
+        w[x] = left - lane > 32 * x ? a.adjwgt[at + 32 * x] : 0;
       }
 #pragma unroll
       for (i32 x = 0; x < kU; ++x) lu[x] = u[x] >= 0 ? a.pos[u[x]] - o : -1;

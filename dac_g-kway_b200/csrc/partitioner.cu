@@ -32,7 +32,7 @@ constexpr i32 kValidateLong = 512;
 __device__ __forceinline__ i32 validate_entries(i32 v, i32 n, i32 b, i32 e, i32 first, i32 step,
                                                 const i32* __restrict__ adjncy, const i32* __restrict__ adjwgt) {
   i32 f = 0;
-  for (i32 j = b + first; j < e; j += step) {
+  for (u32 j = (u32)b + first; j < (u32)e; j += step) {
     const i32 u = adjncy[j];
     if (u < 0 || u >= n) f |= 2;
     else if (u == v) f |= 4;
@@ -67,9 +67,9 @@ __global__ void __launch_bounds__(256) k_validate(i32 n, i64 m, i32 R, const i32
     if (isl) longlist[atomicAdd(longcnt, 1)] = (i32)v;
     if (!__any_sync(0xffffffffu, isl)) {
       const i32 rows = (i32)(n - v0 < R ? n - v0 : R);
-      const i32 end = __shfl_sync(0xffffffffu, e, rows - 1);
+      const u32 end = (u32)__shfl_sync(0xffffffffu, e, rows - 1);
       constexpr int U = 4;
-      for (i32 j0 = __shfl_sync(0xffffffffu, b, 0) + lane0; j0 < end; j0 += 32 * U) {
+      for (u32 j0 = (u32)__shfl_sync(0xffffffffu, b, 0) + lane0; j0 < end; j0 += 32 * U) {
         i32 u[U], wt[U];
 #pragma unroll
         for (int x = 0; x < U; ++x) {
@@ -78,10 +78,12 @@ __global__ void __launch_bounds__(256) k_validate(i32 n, i64 m, i32 R, const i32
         }
 #pragma unroll
         for (int x = 0; x < U; ++x) {
-          const i32 j = j0 + 32 * x;
+          const u32 j = j0 + 32 * x;
           if (wt[x] < 0) f |= 8;
           if (u[x] < 0 || u[x] >= n) f |= 2;
-          else if ((u64)((i64)u[x] - v0) < (u64)rows && j < end && j >= xadj[u[x]] && j < xadj[u[x] + 1]) f |= 4;
+          else if ((u64)((i64)u[x] - v0) < (u64)rows && j < end && j >= (u32)xadj[u[x]] &&
+                   j < (u32)xadj[u[x] + 1])
+            f |= 4;
         }
       }
     } else {   // the other rows by the warp, one after the other

@@ -400,14 +400,17 @@ __device__ __forceinline__ i32 part_words(i32 k) { return (k + 31) >> 5; }
 
 __device__ __forceinline__ void row_connections(const LevelArgs& a, u32* accb, u32* bits, i32 pb, i32 beg, i32 end,
                                                 i32 first, i32 step) {
-  for (i32 e0 = beg + first; e0 < end; e0 += step * kRowU) {
+  const i32* __restrict__ ra = a.adjncy + beg;   // (a row has at most half of the entries: its places are i32)
+  const i32* __restrict__ rw = a.adjwgt + beg;
+  const i32 len = end - beg;
+  for (i32 e0 = first; e0 < len; e0 += step * kRowU) {
     i32 q[kRowU];
     u32 w[kRowU];
 #pragma unroll
     for (i32 x = 0; x < kRowU; ++x) {
       const i32 e = e0 + x * step;
-      q[x] = e < end ? a.adjncy[e] : -1;
-      w[x] = e < end ? (u32)a.adjwgt[e] : 0u;
+      q[x] = e < len ? ra[e] : -1;
+      w[x] = e < len ? (u32)rw[e] : 0u;
     }
 #pragma unroll
     for (i32 x = 0; x < kRowU; ++x) q[x] = q[x] >= 0 ? ldc(a.part + q[x]) : -1;
@@ -565,8 +568,8 @@ __device__ void ph_update_rows(const LevelArgs& a, u32* acc_all, u32* bits_all, 
     u32 g = 0, q_best = (u32)p;
     bool b;
     if (end - beg <= 64) {   // warp-uniform: the row's part ids stay in registers (one load chain)
-      const i32 e0 = beg + lane, e1 = e0 + 32;
-      const bool h0 = e0 < end, h1 = e1 < end;
+      const u32 e0 = (u32)beg + lane, e1 = e0 + 32;
+      const bool h0 = e0 < (u32)end, h1 = e1 < (u32)end;
       const i32 u0 = h0 ? a.adjncy[e0] : 0, u1 = h1 ? a.adjncy[e1] : 0;
       const u32 w0 = h0 ? (u32)a.adjwgt[e0] : 0u, w1 = h1 ? (u32)a.adjwgt[e1] : 0u;
       const i32 q0 = h0 ? ldc(a.part + u0) : p, q1 = h1 ? ldc(a.part + u1) : p;
@@ -612,7 +615,7 @@ __device__ void ph_update_rows(const LevelArgs& a, u32* acc_all, u32* bits_all, 
       continue;
     }
     bool bl = false;
-    for (i32 e = beg + lane; e < end; e += 32) {
+    for (u32 e = (u32)beg + lane; e < (u32)end; e += 32) {
       const i32 q = ldc(a.part + a.adjncy[e]);
       atomicAdd(&accb[q], (u32)a.adjwgt[e]);
       bl |= (q != p);
@@ -622,7 +625,7 @@ __device__ void ph_update_rows(const LevelArgs& a, u32* acc_all, u32* bits_all, 
     if (b) {
       const u32 id = accb[p];
       u64 best = 0;
-      for (i32 e = beg + lane; e < end; e += 32) {
+      for (u32 e = (u32)beg + lane; e < (u32)end; e += 32) {
         const i32 q = ldc(a.part + a.adjncy[e]);
         if (q != p) {
           const u64 key = ((u64)(accb[q] - id) << 32) | (u32)(~(u32)q);
@@ -644,7 +647,7 @@ __device__ void ph_update_rows(const LevelArgs& a, u32* acc_all, u32* bits_all, 
       }
     }
     __syncwarp();
-    for (i32 e = beg + lane; e < end; e += 32) accb[ldc(a.part + a.adjncy[e])] = 0;
+    for (u32 e = (u32)beg + lane; e < (u32)end; e += 32) accb[ldc(a.part + a.adjncy[e])] = 0;
     __syncwarp();
   }
   if (count && lane == 0 && rows) atomicAdd(reinterpret_cast<unsigned long long*>(&st->rows), rows);
@@ -745,13 +748,13 @@ __device__ void ph_update_first_groups(const LevelArgs& a, u32* rows, u32* acc_a
     }
     u32* accb = acc - (act ? part_base_of(a, v) : 0);   // rows are indexed by the graph's own part ids
     // entries sub and sub + G keep their part ids in registers; longer rows reload
-    const i32 e0 = beg + sub, e1 = e0 + G;
-    const bool h0 = e0 < end, h1 = e1 < end;
+    const u32 e0 = (u32)beg + sub, e1 = e0 + G;
+    const bool h0 = e0 < (u32)end, h1 = e1 < (u32)end;
     const i32 q0 = h0 ? ldc(a.part + a.adjncy[e0]) : p, q1 = h1 ? ldc(a.part + a.adjncy[e1]) : p;
     bool bl = q0 != p || q1 != p;
     if (h0) atomicAdd(&accb[q0], (u32)a.adjwgt[e0]);
     if (h1) atomicAdd(&accb[q1], (u32)a.adjwgt[e1]);
-    for (i32 e = e1 + G; e < end; e += G) {
+    for (u32 e = e1 + G; e < (u32)end; e += G) {
       const i32 q = ldc(a.part + a.adjncy[e]);
       atomicAdd(&accb[q], (u32)a.adjwgt[e]);
       bl |= q != p;
@@ -766,7 +769,7 @@ __device__ void ph_update_first_groups(const LevelArgs& a, u32* rows, u32* acc_a
         const u64 key = ((u64)(accb[q1] - id) << 32) | (u32)(~(u32)q1);
         best = best > key ? best : key;
       }
-      for (i32 e = e1 + G; e < end; e += G) {
+      for (u32 e = e1 + G; e < (u32)end; e += G) {
         const i32 q = ldc(a.part + a.adjncy[e]);
         if (q != p) {
           const u64 key = ((u64)(accb[q] - id) << 32) | (u32)(~(u32)q);
@@ -795,7 +798,7 @@ __device__ void ph_update_first_groups(const LevelArgs& a, u32* rows, u32* acc_a
     __syncwarp();
     if (h0) accb[q0] = 0;
     if (h1) accb[q1] = 0;
-    for (i32 e = e1 + G; e < end; e += G) accb[ldc(a.part + a.adjncy[e])] = 0;
+    for (u32 e = e1 + G; e < (u32)end; e += G) accb[ldc(a.part + a.adjncy[e])] = 0;
     __syncwarp();
   }
   update_listed_rows(a, acc_all, bits_all, S, L);
@@ -893,12 +896,13 @@ __device__ u32 ph_candidates(const LevelArgs& a, i32* s_cnt, i32* s_base, u32* s
       bool blocked = false;
       u32 done = 0;   // lanes of blocked rows
       const int first = lane & ~(kIndLanes - 1);   // the row's first lane
-      for (i32 e0 = beg + lane - first; __any_sync(kFullMask, e0 < end && !((done >> first) & kIndMask));
-           e0 += kIndLanes * kIndU) {
+      i64 at = (i64)beg + (lane - first);
+      for (i32 left = end - beg - (lane - first); __any_sync(kFullMask, left > 0 && !((done >> first) & kIndMask));
+           left -= kIndLanes * kIndU, at += kIndLanes * kIndU) {
         i32 u[kIndU], gu[kIndU], tu[kIndU];
         u32 vu[kIndU];
 #pragma unroll
-        for (i32 x = 0; x < kIndU; ++x) u[x] = e0 + kIndLanes * x < end ? a.adjncy[e0 + kIndLanes * x] : INT_MAX;
+        for (i32 x = 0; x < kIndU; ++x) u[x] = left > kIndLanes * x ? a.adjncy[at + kIndLanes * x] : INT_MAX;
 #pragma unroll
         for (i32 x = 0; x < kIndU; ++x) {
           gu[x] = 0;
@@ -925,13 +929,11 @@ __device__ u32 ph_candidates(const LevelArgs& a, i32* s_cnt, i32* s_base, u32* s
       bool blocked = false;
       {   // kRowU entries a lane together, until a lane is blocked
         bool any = false;
-        for (i32 b0 = beg; b0 < end && !any; b0 += 32 * kRowU) {
+        i64 at = (i64)beg + lane;
+        for (i32 left = end - beg; left > 0 && !any; left -= 32 * kRowU, at += 32 * kRowU) {   // (warp-uniform)
           i32 u[kRowU], gu[kRowU];
 #pragma unroll
-          for (i32 x = 0; x < kRowU; ++x) {
-            const i32 e = b0 + 32 * x + lane;
-            u[x] = e < end ? a.adjncy[e] : INT_MAX;
-          }
+          for (i32 x = 0; x < kRowU; ++x) u[x] = left - lane > 32 * x ? a.adjncy[at + 32 * x] : INT_MAX;
 #pragma unroll
           for (i32 x = 0; x < kRowU; ++x) gu[x] = u[x] < cv ? ldc(a.gain + u[x]) : 0;
 #pragma unroll
@@ -1856,10 +1858,11 @@ __device__ void ph_select_batch(const LevelArgs& a, u64* s, i32* greedy, u64* s_
 __device__ __forceinline__ void mark_row(const LevelArgs& a, UStage& S, i32 beg, i32 end) {
   const int lane = threadIdx.x & 31;
   constexpr i32 kU = 4;
-  for (i32 e0 = beg + lane; e0 < end; e0 += 32 * kU) {
+  i64 at = (i64)beg + lane;
+  for (i32 left = end - beg - lane; left > 0; left -= 32 * kU, at += 32 * kU) {
     i32 u[kU], was[kU];
 #pragma unroll
-    for (i32 x = 0; x < kU; ++x) u[x] = e0 + 32 * x < end ? a.adjncy[e0 + 32 * x] : -1;
+    for (i32 x = 0; x < kU; ++x) u[x] = left > 32 * x ? a.adjncy[at + 32 * x] : -1;
 #pragma unroll
     for (i32 x = 0; x < kU; ++x) was[x] = u[x] >= 0 ? atomicExch(&a.updflag[u[x]], 1) : 1;
 #pragma unroll
@@ -2376,7 +2379,7 @@ __device__ void ph_bal_eval(const LevelArgs& a, u32* acc_all, u32* bits_all) {
       __syncwarp();
       row_connections(a, accb, bits, pb, beg, end, lane, 32);
     } else {
-      for (i32 e = beg + lane; e < end; e += 32) atomicAdd(&accb[ldc(a.part + a.adjncy[e])], (u32)a.adjwgt[e]);
+      for (u32 e = (u32)beg + lane; e < (u32)end; e += 32) atomicAdd(&accb[ldc(a.part + a.adjncy[e])], (u32)a.adjwgt[e]);
     }
     __syncwarp();
     const u32 id = accb[p];
@@ -2391,7 +2394,7 @@ __device__ void ph_bal_eval(const LevelArgs& a, u32* acc_all, u32* bits_all) {
       for (i32 ql = lane; ql < a.kacc; ql += 32)
         if ((bits[ql >> 5] >> (ql & 31)) & 1u) consider(pb + ql);
     } else {
-      for (i32 e = beg + lane; e < end; e += 32) consider(ldc(a.part + a.adjncy[e]));
+      for (u32 e = (u32)beg + lane; e < (u32)end; e += 32) consider(ldc(a.part + a.adjncy[e]));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -2415,7 +2418,7 @@ __device__ void ph_bal_eval(const LevelArgs& a, u32* acc_all, u32* bits_all) {
     if (by_parts)
       for (i32 ql = lane; ql < a.kacc; ql += 32) acc[ql] = 0;
     else
-      for (i32 e = beg + lane; e < end; e += 32) accb[ldc(a.part + a.adjncy[e])] = 0;
+      for (u32 e = (u32)beg + lane; e < (u32)end; e += 32) accb[ldc(a.part + a.adjncy[e])] = 0;
     __syncwarp();
   }
 }
@@ -2436,14 +2439,12 @@ __device__ void ph_bal_emit(const LevelArgs& a) {
     const i32 beg = a.xadj[v], end = a.xadj[v + 1];
     bool emit = true;
     constexpr i32 kU = 4;
-    for (i32 b0 = beg; b0 < end && emit; b0 += 32 * kU) {
+    i64 at = (i64)beg + lane;
+    for (i32 left = end - beg; left > 0 && emit; left -= 32 * kU, at += 32 * kU) {   // (warp-uniform)
       i32 u[kU];
       bool yields = false;
 #pragma unroll
-      for (i32 x = 0; x < kU; ++x) {
-        const i32 e = b0 + 32 * x + lane;
-        u[x] = e < end ? a.adjncy[e] : INT_MAX;
-      }
+      for (i32 x = 0; x < kU; ++x) u[x] = left - lane > 32 * x ? a.adjncy[at + 32 * x] : INT_MAX;
 #pragma unroll
       for (i32 x = 0; x < kU; ++x) yields |= u[x] < v && ldc(a.bmark + u[x]) == ep;
       emit = !__any_sync(kFullMask, yields);
@@ -3046,13 +3047,14 @@ __global__ void __launch_bounds__(256) k_cut_pw(i32 n, const i32* __restrict__ x
   // entries first, first + step, ... of v's row
   auto walk = [&](i32 v, i32 p, i32 b, i32 e1, i32 first, i32 step) {
     constexpr i32 kU = 4;
-    for (i32 e0 = b + first; e0 < e1; e0 += step * kU) {
+    i64 at = (i64)b + first;
+    for (i32 left = e1 - b - first; left > 0; left -= step * kU, at += step * kU) {
       i32 u[kU];
 #pragma unroll
-      for (i32 x = 0; x < kU; ++x) u[x] = e0 + x * step < e1 ? adjncy[e0 + x * step] : -1;
+      for (i32 x = 0; x < kU; ++x) u[x] = left > x * step ? adjncy[at + x * step] : -1;
 #pragma unroll
       for (i32 x = 0; x < kU; ++x)
-        if (v < u[x] && part[u[x]] != p) c += (u32)adjwgt[e0 + x * step];
+        if (v < u[x] && part[u[x]] != p) c += (u32)adjwgt[at + x * step];
     }
   };
   const i64 step = ((i64)gridDim.x * blockDim.x) / G;
