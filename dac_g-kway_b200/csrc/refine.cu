@@ -1858,11 +1858,12 @@ __device__ void ph_select_batch(const LevelArgs& a, u64* s, i32* greedy, u64* s_
 __device__ __forceinline__ void mark_row(const LevelArgs& a, UStage& S, i32 beg, i32 end) {
   const int lane = threadIdx.x & 31;
   constexpr i32 kU = 4;
-  i64 at = (i64)beg + lane;
-  for (i32 left = end - beg - lane; left > 0; left -= 32 * kU, at += 32 * kU) {
+  const i32* __restrict__ row = a.adjncy + beg;
+  const i32 len = end - beg;
+  for (i32 e0 = lane; e0 < len; e0 += 32 * kU) {
     i32 u[kU], was[kU];
 #pragma unroll
-    for (i32 x = 0; x < kU; ++x) u[x] = left > 32 * x ? a.adjncy[at + 32 * x] : -1;
+    for (i32 x = 0; x < kU; ++x) u[x] = e0 + 32 * x < len ? row[e0 + 32 * x] : -1;
 #pragma unroll
     for (i32 x = 0; x < kU; ++x) was[x] = u[x] >= 0 ? atomicExch(&a.updflag[u[x]], 1) : 1;
 #pragma unroll
