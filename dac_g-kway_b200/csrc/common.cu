@@ -676,9 +676,10 @@ void forget_coop_event(Handle& h) {
 // Host memory.  A copy from pageable memory is staged by the driver on the
 // calling thread (11.5 GB/s); here several threads fill pinned slots of 2 MB
 // and queue one copy each, which the link takes at 40 GB/s and more: a batch
-// of 256 graphs (349 MB) 65 -> 46 ms.  Small copies and pinned, managed or
-// device pointers take the plain call.  The buffer also holds a graph file's
-// text: pinning memory for each 3.5 MB file cost 2.4 of its 3.7 ms.
+// of 256 graphs (349 MB) 65 -> 46 ms.  Small copies, pinned, managed or device
+// pointers and the per-thread default stream take the plain call.  The buffer
+// also holds a graph file's text: pinning memory for each 3.5 MB file cost 2.4
+// of its 3.7 ms.
 // ---------------------------------------------------------------------------
 constexpr size_t kStageMin = size_t(8) << 20;   // below this the threads cost more than they save
 
@@ -734,6 +735,13 @@ static bool stage_slots(Handle& h) {
   return true;
 }
 
+// Whether this call's copies can be queued by several threads: the per-thread
+// default stream names another stream on each of them, and copies queued there
+// would not be ordered with the caller's kernels.
+static bool staged(const Handle& h, size_t bytes, int threads) {
+  return bytes >= kStageMin && threads >= 2 && h.stream != cudaStreamPerThread;
+}
+
 // Runs work(t) on T threads (this one included) with the handle's device
 // current; returns the first CUDA error.
 template <class Work>
@@ -764,7 +772,7 @@ static int stage_threads() {
 
 void copy_to_device(Handle& h, void* dst, const void* src, size_t bytes) {
   const int T = stage_threads();
-  if (bytes < kStageMin || T < 2 || !pageable(src) || !stage_slots(h)) {
+  if (!staged(h, bytes, T) || !pageable(src) || !stage_slots(h)) {
     if (bytes) GKW_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h.stream));
     return;
   }
@@ -793,7 +801,7 @@ void copy_to_device(Handle& h, void* dst, const void* src, size_t bytes) {
 
 void copy_to_host(Handle& h, void* dst, const void* src, size_t bytes) {
   const int T = stage_threads();
-  if (bytes < kStageMin || T < 2 || !pageable(dst) || !stage_slots(h)) {
+  if (!staged(h, bytes, T) || !pageable(dst) || !stage_slots(h)) {
     if (bytes) GKW_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h.stream));
     GKW_CUDA(cudaStreamSynchronize(h.stream));
     return;
