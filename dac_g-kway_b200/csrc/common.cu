@@ -683,6 +683,55 @@ void forget_coop_event(Handle& h) {
 // ---------------------------------------------------------------------------
 constexpr size_t kStageMin = size_t(8) << 20;   // below this the threads cost more than they save
 
+// All handles of the process together keep at most kStageProcess bytes of
+// buffers and run at most kStageHelpers threads beside their callers (a server
+// has up to 256 slots).  A call that gets neither is an ordinary copy, or pins
+// memory of its own for a file.
+constexpr size_t kStageProcess = 4 * kStageBytes;
+constexpr int kStageHelpers = 28;
+static std::mutex g_stage_mu;
+static size_t g_stage_bytes = 0;
+static int g_stage_helpers = 0;
+
+bool stage_reserve(size_t bytes) {
+  std::lock_guard<std::mutex> lk(g_stage_mu);
+  if (bytes > kStageProcess - g_stage_bytes) return false;
+  g_stage_bytes += bytes;
+  return true;
+}
+
+void stage_unreserve(size_t bytes) {
+  std::lock_guard<std::mutex> lk(g_stage_mu);
+  g_stage_bytes -= bytes;
+}
+
+int stage_take_helpers(int want) {
+  const int all = std::min<int>(kStageHelpers, (int)(std::thread::hardware_concurrency() / 2));
+  std::lock_guard<std::mutex> lk(g_stage_mu);
+  const int n = std::max(0, std::min(want, all - g_stage_helpers));
+  g_stage_helpers += n;
+  return n;
+}
+
+void stage_return_helpers(int n) {
+  std::lock_guard<std::mutex> lk(g_stage_mu);
+  g_stage_helpers -= n;
+}
+
+// The helpers of one copy: up to seven, given back when it ends.
+struct StageHelpers {
+  int n;
+  StageHelpers() : n(0) {}
+  ~StageHelpers() {
+    if (n) stage_return_helpers(n);
+  }
+  static int most() { return std::min(8, (int)(std::thread::hardware_concurrency() / 2)) - 1; }
+  bool take() {
+    n = stage_take_helpers(most());
+    return n > 0;
+  }
+};
+
 static bool pageable(const void* p) {
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
@@ -698,21 +747,29 @@ void free_stage(Handle& h) {
     e = nullptr;
   }
   if (h.stage) cudaFreeHost(h.stage);
+  if (h.stage_cap) stage_unreserve(h.stage_cap);
   h.stage = nullptr;
   h.stage_cap = 0;
 }
 
 char* stage_buffer(Handle& h, size_t bytes) {
   if (bytes > kStageBytes) return nullptr;
-  GKW_CUDA(cudaStreamSynchronize(h.stream));   // copies out of the old contents
-  if (h.stage_cap < bytes) {
+  const bool grow = h.stage_cap < bytes;
+  // small files keep a small buffer; a staged copy needs all the slots
+  size_t cap = size_t(1) << 20;
+  while (cap < bytes) cap <<= 1;
+  if (grow && !stage_reserve(cap)) return nullptr;
+  const cudaError_t e = cudaStreamSynchronize(h.stream);   // copies out of the old contents
+  if (e != cudaSuccess) {
+    if (grow) stage_unreserve(cap);
+    GKW_CUDA(e);
+  }
+  if (grow) {
     free_stage(h);
-    // small files keep a small buffer; a staged copy needs all the slots
-    size_t cap = size_t(1) << 20;
-    while (cap < bytes) cap <<= 1;
     if (cudaHostAlloc((void**)&h.stage, cap, cudaHostAllocDefault) != cudaSuccess) {
       cudaGetLastError();
       h.stage = nullptr;
+      stage_unreserve(cap);
       return nullptr;
     }
     h.stage_cap = cap;
@@ -738,8 +795,8 @@ static bool stage_slots(Handle& h) {
 // Whether this call's copies can be queued by several threads: the per-thread
 // default stream names another stream on each of them, and copies queued there
 // would not be ordered with the caller's kernels.
-static bool staged(const Handle& h, size_t bytes, int threads) {
-  return bytes >= kStageMin && threads >= 2 && h.stream != cudaStreamPerThread;
+static bool staged(const Handle& h, size_t bytes) {
+  return bytes >= kStageMin && StageHelpers::most() > 0 && h.stream != cudaStreamPerThread;
 }
 
 // Runs work(t) on T threads (this one included) with the handle's device
@@ -765,17 +822,13 @@ static cudaError_t on_threads(Handle& h, int T, Work work) {
   return cudaSuccess;
 }
 
-static int stage_threads() {
-  const unsigned hw = std::thread::hardware_concurrency();
-  return (int)std::max(1u, std::min(8u, hw / 2));
-}
-
 void copy_to_device(Handle& h, void* dst, const void* src, size_t bytes) {
-  const int T = stage_threads();
-  if (!staged(h, bytes, T) || !pageable(src) || !stage_slots(h)) {
+  StageHelpers helpers;
+  if (!staged(h, bytes) || !pageable(src) || !stage_slots(h) || !helpers.take()) {
     if (bytes) GKW_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h.stream));
     return;
   }
+  const int T = 1 + helpers.n;
   const size_t nchunk = (bytes + kStageChunk - 1) / kStageChunk;
   const int per = Handle::kStageSlots / T;   // slots of a thread
   const cudaError_t e = on_threads(h, T, [&](int t) {
@@ -800,12 +853,13 @@ void copy_to_device(Handle& h, void* dst, const void* src, size_t bytes) {
 }
 
 void copy_to_host(Handle& h, void* dst, const void* src, size_t bytes) {
-  const int T = stage_threads();
-  if (!staged(h, bytes, T) || !pageable(dst) || !stage_slots(h)) {
+  StageHelpers helpers;
+  if (!staged(h, bytes) || !pageable(dst) || !stage_slots(h) || !helpers.take()) {
     if (bytes) GKW_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h.stream));
     GKW_CUDA(cudaStreamSynchronize(h.stream));
     return;
   }
+  const int T = 1 + helpers.n;
   const size_t nchunk = (bytes + kStageChunk - 1) / kStageChunk;
   const int per = Handle::kStageSlots / T;
   const cudaError_t e = on_threads(h, T, [&](int t) {

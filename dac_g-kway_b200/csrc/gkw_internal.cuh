@@ -231,9 +231,16 @@ void ensure_timer_events(Handle& h);
 constexpr size_t kStageChunk = size_t(2) << 20;
 constexpr size_t kStageBytes = kStageChunk * Handle::kStageSlots;   // 32 MB
 // A pinned buffer of at least `bytes` that the handle keeps, or null above
-// kStageBytes.  Valid until the next staged copy or stage_buffer call.
+// kStageBytes or the process's limit.  Valid until the next staged copy or
+// stage_buffer call.
 char* stage_buffer(Handle& h, size_t bytes);
 void free_stage(Handle& h);
+// The process's share of that: bytes of all handles' buffers, and threads that
+// copies run beside their callers (stage_take_helpers gives up to `want`).
+bool stage_reserve(size_t bytes);
+void stage_unreserve(size_t bytes);
+int stage_take_helpers(int want);
+void stage_return_helpers(int n);
 // Host-to-device copy on the handle's stream.  Large pageable sources go
 // through the pinned slots, filled by several threads; the source is free
 // when the call returns, the copy itself may still be queued.

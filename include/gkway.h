@@ -17,6 +17,11 @@
  *   - Every call returns a gkw_status; gkw_last_error() gives the message of
  *     the last failure on the calling thread.  No C++ exception crosses the ABI.
  *   - A handle is not re-entrant: one host thread per handle at a time.
+ *   - Host arrays of 8 MB and more in pageable memory, and graph files, pass
+ *     through pinned memory that the handle keeps until it is destroyed (up to
+ *     32 MB; 128 MB over all handles and servers of the process), filled and
+ *     emptied by up to 7 short-lived threads beside the caller (28 over the
+ *     process).  Calls beyond these limits copy in the ordinary way.
  */
 #ifndef GKWAY_H_
 #define GKWAY_H_
