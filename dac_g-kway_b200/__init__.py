@@ -498,10 +498,16 @@ class Handle:
         check(lib().gkw_get_tuning(self._h, ctypes.byref(t)))
         return t.as_dict()
 
-    def set_tuning(self, match_lanes=(4, 8, 16, 32), level_verts_per_cta=512, level_min_ctas=32,
-                   coarsen_fused_max_n=0, coarsen_verts_per_cta=256) -> None:
-        t = Tuning((ctypes.c_int32 * 4)(*match_lanes), int(level_verts_per_cta), int(level_min_ctas),
-                   int(coarsen_fused_max_n), int(coarsen_verts_per_cta))
+    def set_tuning(self, match_lanes=None, level_verts_per_cta=None, level_min_ctas=None,
+                   coarsen_fused_max_n=None, coarsen_verts_per_cta=None) -> None:
+        """Sets the named launch shapes; the others stay as the handle has them."""
+        named = {"match_lanes": match_lanes, "level_verts_per_cta": level_verts_per_cta,
+                 "level_min_ctas": level_min_ctas, "coarsen_fused_max_n": coarsen_fused_max_n,
+                 "coarsen_verts_per_cta": coarsen_verts_per_cta}
+        now = self.tuning()
+        now.update({k: v for k, v in named.items() if v is not None})
+        t = Tuning((ctypes.c_int32 * 4)(*now["match_lanes"]), int(now["level_verts_per_cta"]),
+                   int(now["level_min_ctas"]), int(now["coarsen_fused_max_n"]), int(now["coarsen_verts_per_cta"]))
         check(lib().gkw_set_tuning(self._h, ctypes.byref(t)))
 
     def autotune(self, xadj, adjncy, adjwgt, vwgt, k: int, opts: Options | None = None) -> dict:
