@@ -133,6 +133,7 @@ struct CountBarrier {
 };
 
 constexpr int kPinnedWords = 1024;   // Handle::h_pinned
+constexpr gkw_tuning kDefaultTuning{{2, 8, 16, 32}, 128, 16, 0, 256};
 
 // Device-side state of one handle shared by the cooperative kernels and the
 // per-level scalars read back once per level.
@@ -210,7 +211,7 @@ struct Handle {
   // thread-block cluster (a server's small jobs; see launch_coop)
   bool narrow = false;
   cudaEvent_t coop_ev = nullptr;   // this handle's last wide cooperative launch
-  gkw_tuning tuning{{2, 8, 16, 32}, 128, 16, 0, 256};   // launch shapes (gkw_autotune)
+  gkw_tuning tuning = kDefaultTuning;   // launch shapes (gkw_autotune)
   // Pinned staging for pageable host memory and files (copy_to_device and
   // stage_buffer, common.cu): made on first use, at most kStageBytes, freed
   // with the handle

@@ -505,15 +505,29 @@ void partition_multi_impl(Handle& h, const DevGraph& g0, i32 nk, const i32* ks, 
 // its time, so each candidate is timed on a full partition of the caller's
 // graph:
 //   * match lanes: one partition during which every level's match is also
-//     run with 4, 8, 16 and 32 lanes per vertex (best of three launches each,
-//     CUDA events); each average-degree bucket met keeps the lane count with
-//     the least summed time;
-//   * level-kernel density: vertices per CTA in {256, 512, 1024, 2048} x
-//     minimum CTAs in {16, 32, 64}, best of two partitions each by the
-//     refinement phase's event time;
-//   * coarsening: per-phase kernels on every level, or one fused launch per
-//     level for levels of at most 80k or 300k vertices, best of two
-//     partitions each by the coarsening phase's event time.
+//     run with 2, 4, 8, 16 and 32 lanes per vertex (best of three launches
+//     each, CUDA events); each average-degree bucket met keeps the lane count
+//     with the least summed time;
+//   * level-kernel density: the handle's own, then vertices per CTA in
+//     kTuneVerts x minimum CTAs in kTuneMinCtas, best of two partitions each by
+//     the refinement phase's event time;
+//   * coarsening: as the handle has it, then per-phase kernels on every level,
+//     or one fused launch per level for levels of at most 80k or 300k vertices,
+//     best of two partitions each by the coarsening phase's event time.
+constexpr i32 kTuneVerts[] = {128, 256, 512, 1024, 2048};
+constexpr i32 kTuneMinCtas[] = {16, 32, 64};
+constexpr i32 kTuneFused[] = {0, 80000, 300000};
+template <int N>
+constexpr bool among(const i32 (&list)[N], i32 x) {
+  for (i32 y : list)
+    if (x == y) return true;
+  return false;
+}
+static_assert(among(kTuneVerts, kDefaultTuning.level_verts_per_cta) &&
+                  among(kTuneMinCtas, kDefaultTuning.level_min_ctas) &&
+                  among(kTuneFused, kDefaultTuning.coarsen_fused_max_n),
+              "the defaults are candidates of the tuner");
+
 void autotune(Handle& h, const DevGraph& g, i32 k, const gkw_options& opt) {
   i32* part = nullptr;
   GKW_CUDA(cudaMalloc((void**)&part, sizeof(i32) * std::max(g.n, 1)));
@@ -545,39 +559,42 @@ void autotune(Handle& h, const DevGraph& g, i32 k, const gkw_options& opt) {
       if (h.tune_match_ms[b][q] > 0 && (best < 0 || h.tune_match_ms[b][q] < h.tune_match_ms[b][best])) best = q;
     if (best >= 0) h.tuning.match_lanes[b] = lanes[best];
   }
-  gkw_tuning best = h.tuning;
-  double best_ms = 1e300;
-  for (i32 vpc : {256, 512, 1024, 2048}) {
-    for (i32 minc : {16, 32, 64}) {
-      h.tuning.level_verts_per_cta = vpc;
-      h.tuning.level_min_ctas = minc;
-      double t = 1e300;
-      for (int rep = 0; rep < 2; ++rep) {
-        run(&st);
-        t = std::min(t, st.ms_refine);
-      }
-      if (t < best_ms) {
-        best_ms = t;
-        best = h.tuning;
-      }
-    }
-  }
-  h.tuning = best;
-  // coarsening: the per-phase kernels, or one fused launch for the levels of
-  // at most 80k / 300k vertices, by the coarsening phase's event time
-  best_ms = 1e300;
-  for (i32 fmax : {0, 80000, 300000}) {
-    h.tuning.coarsen_fused_max_n = fmax;
-    h.tuning.coarsen_verts_per_cta = 256;
+  // the handle's own shapes first: a candidate has to beat them
+  auto timed = [&](double gkw_stats::* phase) {
     double t = 1e300;
     for (int rep = 0; rep < 2; ++rep) {
       run(&st);
-      t = std::min(t, st.ms_coarsen);
+      t = std::min(t, st.*phase);
     }
+    return t;
+  };
+  const gkw_tuning own = h.tuning;
+  gkw_tuning best = own;
+  double best_ms = timed(&gkw_stats::ms_refine);
+  auto keep_if_faster = [&](double gkw_stats::* phase) {
+    const double t = timed(phase);
     if (t < best_ms) {
       best_ms = t;
       best = h.tuning;
     }
+  };
+  for (i32 vpc : kTuneVerts) {
+    for (i32 minc : kTuneMinCtas) {
+      if (vpc == own.level_verts_per_cta && minc == own.level_min_ctas) continue;
+      h.tuning.level_verts_per_cta = vpc;
+      h.tuning.level_min_ctas = minc;
+      keep_if_faster(&gkw_stats::ms_refine);
+    }
+  }
+  h.tuning = best;
+  // coarsening: as the handle has it, the per-phase kernels, or one fused
+  // launch for the levels of at most 80k / 300k vertices
+  best_ms = timed(&gkw_stats::ms_coarsen);
+  for (i32 fmax : kTuneFused) {
+    if (fmax == own.coarsen_fused_max_n) continue;
+    h.tuning.coarsen_fused_max_n = fmax;
+    h.tuning.coarsen_verts_per_cta = kDefaultTuning.coarsen_verts_per_cta;
+    keep_if_faster(&gkw_stats::ms_coarsen);
   }
   h.tuning = best;
 }
