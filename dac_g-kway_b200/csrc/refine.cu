@@ -325,8 +325,13 @@ __device__ void ph_project(const LevelArgs& a, UStage& S) {
   if (threadIdx.x == 0) S.cnt = 0;
   __syncthreads();
   const i64 stride = (i64)gridDim.x * blockDim.x;
+  // entries in the stage, counted at the barriers: a warp that is ahead may be
+  // appending the next chunk while another has still to decide on the flush, so
+  // the decision does not read S.cnt
+  i32 have = 0;
   for (i64 b0 = (i64)blockIdx.x * blockDim.x; b0 < a.n; b0 += stride) {   // block-uniform trip count
     const i64 v = b0 + threadIdx.x;
+    bool b = false;
     if (v < a.n) {
       const i32 c = a.cmap[v];
       i32 p, bc;
@@ -344,18 +349,19 @@ __device__ void ph_project(const LevelArgs& a, UStage& S) {
       a.gain[v] = 0;
       a.target[v] = p;
       a.inP[v] = 0;
-      const bool b = bc != 0 && !enter && (!a.batch || __ldg(a.gflags + __ldg(a.gid + v)) != 0);
+      b = bc != 0 && !enter && (!a.batch || __ldg(a.gflags + __ldg(a.gid + v)) != 0);
       a.updflag[v] = b ? 1 : 0;
       if (b) S.buf[atomicAdd(&S.cnt, 1)] = (i32)v;   // room: flushed below once half full
     }
-    __syncthreads();
-    if (S.cnt > kUStage - (i32)blockDim.x) {   // block-uniform
-      if (threadIdx.x == 0) S.base = atomicAdd(&a.st->ucount, S.cnt);
+    have += __syncthreads_count(b);
+    if (have > kUStage - (i32)blockDim.x) {   // block-uniform
+      if (threadIdx.x == 0) S.base = atomicAdd(&a.st->ucount, have);
       __syncthreads();
-      for (i32 t = threadIdx.x; t < S.cnt; t += blockDim.x) a.U[S.base + t] = S.buf[t];
+      for (i32 t = threadIdx.x; t < have; t += blockDim.x) a.U[S.base + t] = S.buf[t];
       __syncthreads();
       if (threadIdx.x == 0) S.cnt = 0;
       __syncthreads();
+      have = 0;
     }
   }
   ustage_flush(S, a.U, &a.st->ucount);
