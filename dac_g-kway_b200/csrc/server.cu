@@ -465,14 +465,27 @@ int64_t gkw_predict_footprint(int32_t n, int64_t nnz, int32_t k) {
   // from the allocations of the pipeline: the input and output arrays, the
   // coarser levels (each level keeps at most ~0.6 of the vertices and entries
   // of the level below, so they sum to 1.5x the input), the cmaps, the
-  // refinement state, and the coarsening scratch of the largest level
-  const double nn = std::max<int32_t>(n, 1), mm = (double)std::max<int64_t>(nnz, 1);
+  // refinement state, and the largest scratch of any phase.
+  // Components never merge: with m / 2 edges at least n - m / 2 vertices stay
+  // on every level and reach the initial partition, which otherwise has about
+  // the coarsening threshold's 20 a part.
+  const double nn = std::max<int32_t>(n, 1), mm = (double)std::max<int64_t>(nnz, 1), kk = std::max(k, 1);
+  const double stay = std::max(0.0, nn - 0.5 * mm);
+  const double coarsest = std::min(nn, std::max(stay, 20.0 * kk));
   const double input = 4.0 * (nn + 1) + 8.0 * mm + 8.0 * nn;
-  const double coarse = 1.5 * (12.0 * nn + 8.0 * mm) + 2.5 * 4.0 * nn;
-  const double refine = 96.0 * nn + 32.0 * (double)std::max(k, 1);
-  const double scratch = 64.0 * nn + 24.0 * mm;
+  // (matched vertices at least halve, so there are at most log2 of them levels)
+  const double levels = 1.0 + std::log2(std::min(nn, mm));
+  const double coarse = 1.5 * (12.0 * nn + 8.0 * mm) + 2.5 * 4.0 * nn + 12.0 * stay * std::max(0.0, levels - 2.0);
+  const double refine = 96.0 * nn + 32.0 * kk;
+  // coarsening: the sums, member lists and groups of run_large_level, or the
+  // row tables with the rows (8 an entry), and beside them what the levels'
+  // arrays, allocated for the level below, take beyond the sum above
+  const double coarsening = std::max(88.0 * nn + 8.0 * mm, 64.0 * nn + 24.0 * mm);
+  // initial partition: eight trials' states and 64-bit keys, members, headers,
+  // sides, and the rows
+  const double init = 236.0 * coarsest + 8.0 * mm + 160.0 * kk;
   const double fixed = 16.0 * (1 << 20);
-  return (int64_t)(input + coarse + refine + scratch + fixed);
+  return (int64_t)(input + coarse + refine + std::max(coarsening, init) + fixed);
 }
 
 gkw_status gkw_server_create(gkw_server** out, int32_t device, const gkw_server_config* cfg) {
