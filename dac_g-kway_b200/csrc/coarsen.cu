@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(kUfSmallThreads) k_uf_small(i32 n, const i32* 
   }
   if (threadIdx.x == 0) s_rounds = 0;
   __syncthreads();
-  for (i32 v = threadIdx.x; v < n; v += T)
+  for (i32 v = n - 1 - (i32)threadIdx.x; v >= 0; v -= T)   // (largest first: see k_uf_hook)
     if (cand[v] < v) uf_unite<true>(parent, v, cand[v]);
   __syncthreads();
   for (i32 v = threadIdx.x; v < n; v += T)
@@ -365,10 +365,13 @@ __global__ void k_uf_init(i32 n, const i32* __restrict__ cand, UfStart uf) {
   if (v < n) uf.set((i32)v, cand[v]);
 }
 
+// Largest vertices first: a hub of small id then has its largest leaf as root
+// at once, and every other leaf hangs itself under that, each on its own word;
+// from the smallest up, every leaf raised the root that all of them share.
 __global__ void k_uf_hook(i32 n, const i32* __restrict__ cand, i32* parent, i32* rounds_out) {
-  const i64 v = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+  const i64 v = (i64)n - 1 - ((i64)blockIdx.x * blockDim.x + threadIdx.x);
   if (v == 0) *rounds_out = 0;   // raised by the walk
-  if (v >= n) return;
+  if (v < 0) return;
   const i32 c = cand[v];
   if (c < (i32)v) uf_unite<false>(parent, (i32)v, c);
 }
@@ -838,7 +841,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_group_small(SmallLevel a) {
     *a.maxdeg = 0;
   }
   __syncthreads();
-  for (i32 v = t; v < n; v += T)
+  for (i32 v = n - 1 - t; v >= 0; v -= T)   // (largest first: see k_uf_hook)
     if (cand[v] < v) uf_unite<true>(parent, v, cand[v]);
   __syncthreads();
   for (i32 v = t; v < n; v += T)
