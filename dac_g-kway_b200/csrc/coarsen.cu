@@ -1540,7 +1540,8 @@ __global__ void __launch_bounds__(512) k_contract_cta(
 // kept one warp for 32k (all levels of a 4M-vertex circuit graph: 4.4 ms, now
 // 0.9).  On levels of up to 100k vertices R = 8 (or 4) gives more warps a
 // shorter chain (2048 vertices: 7.6 us, now 5.3; on a million R = 8 is 2.6x
-// slower than 32).
+// slower than 32; the line: coarsening of a 90k mesh 324 us with 32 and 314
+// with 8, of a 130k one the same, of a 200k one 403 and 413).
 // Also the level's longest coarse row and heaviest coarse vertex (both
 // *maxdeg and *max_cvw start at zero).
 __global__ void k_copy_rows(const i32* __restrict__ ncp, i32 R, const i32* __restrict__ ub,
@@ -1825,9 +1826,13 @@ static void contract_rows(Handle& h, const DevGraph& g, const ContractTables& t,
   // Where a row can outgrow the smaller tables, the rows that did go through
   // the 512 one: a level whose mean hides rows of a few hundred entries (a
   // union of 256 circuits and meshes: 120k of them) left those to one CTA each
-  // (5.3 ms on its first level, now 0.84).  Smaller levels have too few such
-  // rows: a warp takes longer over one than a CTA (a 30k-vertex circuit's
-  // coarsening 0.56 ms with a CTA each, 0.81 with warps).
+  // (5.3 ms on its first level, now 0.84).  A warp takes longer over one row
+  // than a CTA, so the pass pays where rows of a few hundred entries are many,
+  // which the host does not know.  By n, coarsening in ms without the pass and
+  // with it: 60k vertices, circuit 0.71 / 0.98, mesh with 1% of hubs of 100
+  // 0.60 / 0.77; 200k, 1.18 / 1.26 and 1.10 / 0.98; 800k, 3.22 / 3.36 and
+  // 2.98 / 2.18: below 100k it loses on both, above it a little on the one and
+  // much less than it gains on the other.
   constexpr i32 kMid512 = 100000;
   i32 *over = heavy, *nover = misc, *free_list = mid;
   i32 W = wide_ids || expL <= 100 ? 128 : expL <= 400 ? 256 : 512;
@@ -1940,7 +1945,7 @@ struct FusedArgs {
   const i32* adjncy;
   const i32* adjwgt;
   const i32* vwgt;
-  i32 lanes;     // match lanes per vertex (4, 8, 16, 32)
+  i32 lanes;     // match lanes per vertex (2, 4, 8, 16, 32)
   i32 split;     // rows above kMatchLong may exist
   i32 cap;       // group cap
   i32 max_rounds;

@@ -179,7 +179,7 @@ struct Handle {
   bool own_stream = false;
   Pool hier;
   Pool scratch;
-  i64* h_pinned = nullptr;      // 64 pinned i64 slots for scalar readbacks
+  i64* h_pinned = nullptr;      // kPinnedWords pinned i64 words for scalar readbacks and reports
   i32 sm_count = 148;
   i32 smem_optin = 232448;      // opt-in shared memory per block of the device
   ScanState* scan = nullptr;    // single-pass scan state
@@ -221,7 +221,7 @@ struct Handle {
   static constexpr int kStageSlots = 16;
   cudaEvent_t stage_ev[kStageSlots] = {};   // last copy out of (or into) each slot
   // while the autotuner collects: per average-degree bucket, the summed time
-  // of each match lane count (4, 8, 16, 32) over the levels met
+  // of each match lane count (2, 4, 8, 16, 32) over the levels met
   bool tune_collect = false;
   double tune_match_ms[4][kMatchLaneChoices] = {};
   Handle() : hier(size_t(256) << 20), scratch(size_t(256) << 20) {}
@@ -290,7 +290,7 @@ inline void launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, c
   count_launch();
 }
 
-// ---- device primitives (scan.cu) ----
+// ---- device primitives (common.cu) ----
 // Exclusive scan of `in` (n entries) into `out` (n entries); if `total` is not
 // null, the grand total is stored there (device pointer).  `in` may equal `out`.
 // d_last (device, may be null): the scan ends with element *d_last, and the

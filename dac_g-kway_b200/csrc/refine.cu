@@ -2153,7 +2153,7 @@ __device__ bool refine_check_risk(const LevelArgs& a, i32 cnt, const RiskLoads& 
 //    every index is balanced, all candidates move, and their order does not
 //    matter: no sort, no check.
 //  * cnt <= cap otherwise: the check over the flagged parts alone, in key
-//    order (refine_threshold); the moves with key <= K* apply.
+//    order (refine_check_risk); the moves with key <= K* apply.
 //  * cnt > cap, or too many events for that check: every CTA that owns a
 //    move index below B sorts the candidates itself (all get the same order)
 //    and runs the check over all parts (refine_balanced_pos).

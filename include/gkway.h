@@ -123,7 +123,7 @@ gkw_status gkw_set_stream(gkw_handle* h, void* stream);
  *                        (b = 0..3; 2, 4, 8, 16 or 32; rows above 512 entries
  *                        always go to one CTA each)
  *   level_verts_per_cta  level-kernel CTAs: one per this many vertices ...
- *   level_min_ctas       ... and at least this many (capped at 2 per SM)
+ *   level_min_ctas       ... and at least this many (capped at one per SM)
  *   coarsen_fused_max_n  coarsening levels of at most this many vertices run
  *                        as one fused launch with grid barriers between the
  *                        phases (default 0: every level as per-phase kernels)
