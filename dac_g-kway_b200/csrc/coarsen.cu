@@ -61,12 +61,14 @@ __global__ void __launch_bounds__(256) k_match(i32 n, const i32* __restrict__ xa
     if (skip) {
       if (sub == 0) longlist[atomicAdd(longcnt, 1)] = v;
     } else {
-      for (u32 e = (u32)beg + sub; e < (u32)end; e += G) {
-        const u32 w = (u32)__ldg(adjwgt + e);
+      const i32 *rw = adjwgt + beg, *ra = adjncy + beg;
+      const i32 len = end - beg;
+      for (i32 e = sub; e < len; e += G) {   // places from the row's start
+        const u32 w = (u32)__ldg(rw + e);
         if (w == 0 || w < bw) continue;
-        const i32 u = __ldg(adjncy + e);
+        const i32 u = __ldg(ra + e);
         const u32 d = (u32)(__ldg(xadj + u + 1) - __ldg(xadj + u));
-        if (w > bw || d < bd) { bw = w; bd = d; bpos = (i32)e; bu = u; }
+        if (w > bw || d < bd) { bw = w; bd = d; bpos = e; bu = u; }
       }
     }
   }
