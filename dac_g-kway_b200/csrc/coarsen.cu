@@ -1010,6 +1010,16 @@ __device__ __forceinline__ u32 hash_u32(u32 x) {
 
 static constexpr u32 kEmpty = 0xffffffffu;
 
+// Slots of a table for a row of L entries: a power of two of at least twice
+// that, 2^31 at most.  (A row of more than 2^30 entries has far fewer distinct
+// ids, one per coarse vertex; doubling on for it would pass 2^32 to zero and
+// never end.)
+__host__ __device__ u32 table_slots(u32 L) {
+  u32 s = 64;
+  while (s < 0x80000000u && s < 2 * (u64)L) s <<= 1;
+  return s;
+}
+
 // Insert (key, w) into an open-addressing table of size hsz (power of two).
 // The table always has free slots (hsz >= 2 * entries), so the probe ends;
 // the probe count is still bounded by hsz.
@@ -1470,8 +1480,7 @@ __global__ void __launch_bounds__(512) k_contract_cta(
     const i32 c = heavy[b];
     const i32 L = rowlen[c];
     const bool global_table = L > cta_cap;   // block-uniform
-    u32 hsz = 64;
-    while (hsz < 2u * (u32)L) hsz <<= 1;
+    const u32 hsz = table_slots((u32)L);
     u32 *keys, *vals;
     u64* out;
     if (global_table) {
@@ -2552,8 +2561,7 @@ __global__ void __launch_bounds__(kFusedThreads, 2) k_coarsen_fused(FusedArgs a)
       const i32 c = ldcg(a.heavy + b);
       const i32 L = ldcg(a.rowlen + c);
       const bool global_table = L > kFusedCtaCap;
-      u32 hsz = 64;
-      while (hsz < 2u * (u32)L) hsz <<= 1;
+      const u32 hsz = table_slots((u32)L);
       u32 *tk, *tv;
       u64* out;
       if (global_table) {
